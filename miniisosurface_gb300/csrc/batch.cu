@@ -5,6 +5,7 @@
 
 #include "batch_kernels.cuh"
 #include "capi_internal.h"
+#include "count_rows.cuh"
 
 using namespace capi;
 
@@ -51,12 +52,12 @@ void replan(iso_ctx* ctx, std::vector<BatchItem>& items, const std::vector<int>&
 // memory before every run and copied in by the first node.
 // ---------------------------------------------------------------------------
 struct FusedGroup {
-    iso::CountVariant cv{};
+    bool aligned = false;      // count: rows a multiple of 4 points
     int rpw = 0, index_bytes = 4;
     std::vector<int> members;  // descriptor indices
     unsigned total = 0;        // blocks (count, scan) or work items (generate)
     size_t list_at = 0, first_at = 0;
-    size_t smem = 0;
+    int stage = 0;             // count: bytes of a warp's buffer, the most of the members
     int ws_bytes = 0;
 };
 
@@ -120,19 +121,19 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
         x.g = g;
         x.gs = iso::make_grad_scale(g);
         x.iso = req[r].isoval;
-        const iso::CountVariant cv = iso::count_variant(g);
-        x.count_KC = std::max(it.pl.cp.KC, kc_min);  // at least 16 planes per block: 157 small grids 2.77 -> 2.72 ms
-        x.count_nyb = (g.ny + 8 * cv.rpw - 1) / (8 * cv.rpw);  // kCountRows warps of cv.rpw rows
+        x.below = iso::count_below(x.iso);
+        const iso::BatchCount bc = iso::batch_count(g, std::max(it.pl.cp.KC, kc_min));
+        x.count_KC = bc.KC;
+        x.count_groups = bc.groups;
         x.nseg = it.pl.cp.nseg;
-        const int ck = cv.rpw | (cv.aligned ? 16 : 0) | (cv.full ? 32 : 0);
-        if (!ckey.count(ck)) {
-            ckey[ck] = (int)f.count.size();
+        if (!ckey.count(bc.aligned)) {
+            ckey[bc.aligned] = (int)f.count.size();
             f.count.emplace_back();
-            f.count.back().cv = cv;
+            f.count.back().aligned = bc.aligned;
         }
-        FusedGroup& cg = f.count[ckey[ck]];
+        FusedGroup& cg = f.count[ckey[bc.aligned]];
         cg.members.push_back(d);
-        cg.smem = std::max(cg.smem, iso::count_batch_smem(g, cv));
+        cg.stage = std::max(cg.stage, bc.stage);
         f.all.members.push_back(d);
         if (extract) {
             const int rpw = iso::gen_rows_per_warp(g.W);
@@ -159,7 +160,7 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
         long long t = 0;
         for (int d : grp.members) {
             const iso::BatchReq& x = f.proto[d];
-            if (what == 0) t += (long long)x.count_nyb * ((x.g.nz + x.count_KC - 1) / x.count_KC);
+            if (what == 0) t += iso::batch_count(x.g, x.count_KC).blocks;
             else if (what == 1) t += x.nseg;
             else t += (long long)x.gen_ngroups * x.gen_nkc;
         }
@@ -187,7 +188,7 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
         for (size_t q = 0; q < m; ++q) {
             fs[q] = run;
             const iso::BatchReq& x = f.proto[grp.members[q]];
-            run += what == 0 ? (unsigned)(x.count_nyb * ((x.g.nz + x.count_KC - 1) / x.count_KC))
+            run += what == 0 ? (unsigned)iso::batch_count(x.g, x.count_KC).blocks
                              : (what == 1 ? (unsigned)x.nseg : (unsigned)(x.gen_ngroups * x.gen_nkc));
         }
         fs[m] = run;
@@ -278,7 +279,7 @@ void enqueue_fused(iso_ctx* ctx, const FusedPlan& f, bool extract, cudaStream_t 
     cudaMemcpyAsync(base, ctx->h_fused, f.upload, cudaMemcpyHostToDevice, s);
     fan_out(ctx, f.count, s, [&](size_t q, cudaStream_t st) {
         const FusedGroup& g = f.count[q];
-        iso::launch_count_batch(g.cv, D, L(g), F(g), (int)g.members.size(), g.total, g.smem, st);
+        iso::launch_count_batch(g.aligned, D, L(g), F(g), (int)g.members.size(), g.total, g.stage, st);
     });
     iso::launch_scan_batch(D, L(f.all), F(f.all), nf, f.all.total, s);
     if (!extract) return;
@@ -431,12 +432,12 @@ std::vector<unsigned char> batch_key(const iso_ctx* ctx, int lanes, int share, c
     for (const std::vector<FusedGroup>* gs : {&fz.count, &fz.gen}) {
         for (const FusedGroup& g : *gs) {
             put(&g.total, sizeof g.total);
-            put(&g.smem, sizeof g.smem);
+            put(&g.stage, sizeof g.stage);
             put(&g.ws_bytes, sizeof g.ws_bytes);
             put(&g.rpw, sizeof g.rpw);
             put(&g.index_bytes, sizeof g.index_bytes);
-            const int cv[3] = {g.cv.rpw, g.cv.aligned ? 1 : 0, g.cv.full ? 1 : 0};  // no padding bytes in the key
-            put(cv, sizeof cv);
+            const int al = g.aligned ? 1 : 0;
+            put(&al, sizeof al);
             put(&g.list_at, sizeof g.list_at);
             put(&g.first_at, sizeof g.first_at);
         }

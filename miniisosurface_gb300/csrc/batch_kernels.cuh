@@ -28,8 +28,8 @@ struct BatchReq {
     long long capV, capT;
     Grid g;
     GradScale gs;
-    float iso;
-    int count_KC, count_nyb;                // count: blocks of count_nyb row blocks x columns of count_KC planes
+    float iso, below;                       // the isovalue and the float below it (count_rows.cuh)
+    int count_KC, count_groups;             // count: items of (row group, run of count_KC planes)
     int nseg;                               // scan segments
     int gen_KC, gen_ngroups, gen_nkc;       // generate: items of (row group, run of gen_KC planes)
 };
@@ -55,18 +55,20 @@ __device__ __forceinline__ int batch_find(const unsigned* __restrict__ first, in
     return lo;
 }
 
-// Count kernel variant of a request: rows per warp (8, 4, 2), row length a multiple of 4 points, and
-// every lane's word inside the row.
-struct CountVariant {
-    int rpw;
-    bool aligned, full;
+// A request's share of the fused count launch: consecutive rows per lane, and its work split for columns of `planes`.
+constexpr int kBatchCountRows = 2;  // 64 uneven volumes, whole call: 2.41 ms, with four 2.48
+struct BatchCount {
+    bool aligned;      // rows a multiple of 4 points: the launch it belongs to
+    int stage;         // bytes of a warp's buffer
+    int groups, KC;
+    long long blocks;
 };
-CountVariant count_variant(const Grid& g);
+BatchCount batch_count(const Grid& g, int planes);
 // Rows per warp of the generate pass (rows of up to 16 words).
 inline int gen_rows_per_warp(int W) { return W <= 4 ? 8 : (W <= 8 ? 4 : 2); }
 
-void launch_count_batch(const CountVariant& v, const BatchReq* reqs, const int* list, const unsigned* first, int m,
-                        unsigned blocks, size_t smem, cudaStream_t s);
+void launch_count_batch(bool aligned, const BatchReq* reqs, const int* list, const unsigned* first, int m,
+                        unsigned blocks, int stage, cudaStream_t s);
 void launch_scan_batch(const BatchReq* reqs, const int* list, const unsigned* first, int m, unsigned blocks,
                        cudaStream_t s);
 void launch_vfirst_batch(const BatchReq* reqs, const int* list, int m, unsigned long long* vfirst, cudaStream_t s);
@@ -81,8 +83,6 @@ void launch_gen_batch(int rpw, int index_bytes, const BatchReq* reqs, const int*
                       cudaStream_t s);
 void launch_vertices_batch(const BatchReq* reqs, const int* list, const unsigned long long* vfirst, int m, int nsm,
                            cudaStream_t s);
-// Shared memory of a count block of the variant (count_buffer_floats for kCountRows warps).
-size_t count_batch_smem(const Grid& g, const CountVariant& v);
 // Shared memory per warp of the generate kernel for rows of W words.
 size_t gen_batch_ws_bytes(int W, int rpw);
 

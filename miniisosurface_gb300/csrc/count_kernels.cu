@@ -2,19 +2,19 @@
 // on sm_103a, with pass 1 (x-edge classification, trims) fused into pass 2
 // (cube cases, per-row counts):
 //
-//   k_count_tma    (rows up to 1024 points, 16-byte aligned) a CTA owns a block
-//   k_count_warps  (up to 2048) of 16 or 32 grid rows (k_count_tma: a half- or
-//                  quarter-warp per row) / 8 rows (k_count_warps: a warp per row) and a run of
-//                  KC planes and marches along z.  Each row's words of plane
-//                  k+1 are classified straight from the volume (plane k+2
-//                  already in flight: a TMA bulk copy into the warp's shared
-//                  buffer, or float4 loads into registers) into bit-per-point
-//                  words held one per lane -- the reference's edgeCases bytes
-//                  are never materialised -- and counted for grid row (j,k): its cut
-//                  x, y and z edges (the vertices it owns), the trims xl/xr,
-//                  the triangles of cell row (j,k) and, for Marching Cubes,
-//                  the vertices cell row (j,k) owns, all 32 cells of a word at
-//                  once (tris_of_word, mc_verts_of_word).  Writes the bit
+//   k_count_rows   (rows up to 1024 points, the volume at a 16-byte boundary;
+//                  count_rows.cuh) a warp owns 1 to 128 neighbouring grid rows
+//                  and a run of KC planes and marches along z, a bulk copy of
+//                  its rows of plane k+2 in flight while plane k is counted.
+//   k_count_warps  (up to 2048 points, any boundary) a CTA owns a block of 8
+//                  grid rows, a warp per row.
+//                  Either way each row's words of plane k+1 are classified
+//                  straight from the volume into bit-per-point words -- the
+//                  reference's edgeCases bytes are never materialised -- and
+//                  counted for grid row (j,k): its cut x, y and z edges (the
+//                  vertices it owns), the trims xl/xr, the triangles of cell
+//                  row (j,k) and, for Marching Cubes, the vertices cell row
+//                  (j,k) owns, all 32 cells of a word at once.  Writes the bit
 //                  words for pass 4.  No warp waits for another.
 //   k_count_wide   rows longer than 2048 points, walked in chunks.
 //   k_scan_*       exclusive scans of the per-row counts in (k, j) order, the
@@ -22,8 +22,9 @@
 //                  vertex of every row (gridEdge xstart and triCounter after
 //                  pass 3) and the totals.
 #include "batch_kernels.cuh"
-#include "count_words.cuh"
+#include "count_rows.cuh"
 #include "iso_kernels.h"
+#include <algorithm>
 
 namespace iso {
 
@@ -196,253 +197,48 @@ __global__ void __launch_bounds__(kThreads) k_count_warps(const float* __restric
     }
 }
 
-// Word wd of a row that starts o floats into a 16-byte aligned buffer and is
-// npts points long, for rows at any offset: the 8 float4 from the one that
-// holds the word's first point (rotated over the lanes as in row_word), the 4
-// points after them from the next lane's word of the same row (lane wd + 1
-// builds its own first float4 from them) or, for the last lane of the row's
-// group (last), by one more load; the 36 bits shifted down by o & 3.  Every
-// lane of the warp calls it (the shuffle); only float4 that hold points of the
-// row are read.
-__device__ __forceinline__ uint32_t row_word_shift(const float* buf, int o, int npts, int wd, int rot, bool last,
-                                                   float iso)
+// Rows of up to 32 words, the volume at a 16-byte boundary (count_rows.cuh).  Against the kernel it replaced (lanes
+// per row a power of two, every row classified twice), us: 768^3 302 / 453, 667 x 228 x 724 94 / 152, 301 x 217 x 190
+// 18.6 / 32, 64^3 10 / 21; 512^3 104 / 103, both at the HBM rate (6.6 TB/s alone; in a sequence of extractions the
+// mesh written before drains at the same time).
+template <bool MC, int S, bool ALIGNED>
+__global__ void __launch_bounds__(kCountThreads) k_count_rows(const float* __restrict__ vol, Grid g, float below,
+                                                              int KC, int ngroups, unsigned nitems, int stage_bytes,
+                                                              uint4* __restrict__ rowcnt,
+                                                              uint2* __restrict__ trims, uint32_t* __restrict__ mccnt,
+                                                              uint32_t* __restrict__ bits_out,
+                                                              unsigned long long* __restrict__ status)
 {
-    const int base = o + 32 * wd, b4 = base >> 2, sh = base & 3;
-    const int nvq = ((o + npts + 3) >> 2) - b4;  // float4 from b4 on that hold points of the row
-    const float4* r4 = reinterpret_cast<const float4*>(buf) + b4;
-    uint32_t w = 0u;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int q = (u + rot) & 7;
-        if (q < nvq) {
-            const float4 v = r4[q];
-            w |= ge_mask(v.x, iso) & (1u << (4 * u));
-            w |= ge_mask(v.y, iso) & (2u << (4 * u));
-            w |= ge_mask(v.z, iso) & (4u << (4 * u));
-            w |= ge_mask(v.w, iso) & (8u << (4 * u));
-        }
-    }
-    w = __funnelshift_l(w, w, 4 * rot);
-    uint32_t hi = __shfl_down_sync(0xffffffffu, w, 1);
-    if (last) {
-        hi = 0u;
-        if (nvq > 8) {
-            const float4 v = r4[8];
-            hi = (ge_mask(v.x, iso) & 1u) | (ge_mask(v.y, iso) & 2u) | (ge_mask(v.z, iso) & 4u) |
-                 (ge_mask(v.w, iso) & 8u);
-        }
-    }
-    const uint32_t r = __funnelshift_r(w, hi, sh);
-    const int nv = npts - 32 * wd;  // points of the word inside the row
-    return nv >= 32 ? r : (nv > 0 ? r & ((1u << nv) - 1u) : 0u);
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ uint64_t s_bar[kCountWarps];
+    const int warp = threadIdx.x >> 5;
+    const unsigned item = blockIdx.x * kCountWarps + warp;
+    if (item >= nitems) return;
+    const FloatSamples<ALIGNED> smp(below);
+    count_rows_item<FloatSamples<ALIGNED>, MC, S>(vol, g, smp, KC, ngroups, item,
+                                                  s_raw + (size_t)warp * stage_bytes,
+                                                  s_bar + warp, rowcnt, trims, mccnt, bits_out, status);
 }
 
-// Floats of a warp's buffer in k_count_tma: RPW + 1 rows (plus up to 3 points
-// of lead-in and padding to 16 bytes when the rows are not 16-byte aligned).
-__host__ __device__ inline int count_buffer_floats(int nx, int rpw, bool aligned)
+// The Flying Edges counts of a list of requests (batch_kernels.cuh), one launch: block x is block x - first[q] of
+// request list[q].
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kCountThreads) k_count_rows_batch(const BatchReq* __restrict__ reqs,
+                                                                    const int* __restrict__ list,
+                                                                    const unsigned* __restrict__ first, int m,
+                                                                    int stage_bytes)
 {
-    return aligned ? (rpw + 1) * nx : (((rpw + 1) * nx + 3) + 3) & ~3;
-}
-
-// Rows of up to 32 words (nx <= 1024), several per warp up to 16 words so
-// that no lane idles on words past a short row: the counts of k_count_warps,
-// with the volume brought in by the TMA bulk engine.  A warp's grid rows
-// jw .. jw+RPW-1 read rows jw .. jw+RPW of every plane (A and B of each
-// row's lanes), which lie next to each other in memory: one cp.async.bulk per
-// plane fills the warp's buffer and completes on the warp's mbarrier.  The
-// words of plane k+1 are taken from the buffer before the copy of plane k+2
-// is issued into it, so the copy runs while step k is counted; no register
-// holds raw values across a step.  Rows whose length is not a multiple of 4
-// points (ALIGNED false; the volume itself 16-byte aligned): the copy runs
-// from the rows' first point rounded down to 16 bytes to their last rounded
-// down, the last few points come by plain loads, and row_word_shift builds
-// the words at the rows' offsets in the buffer.
-// RPW grid rows per warp (1: rows of 17-32 words, 2: up to 16, 4: up to 8, 8: up to 4), LPR =
-// 32 / RPW lanes per row; a warp's rows jw .. jw+RPW-1 read rows jw .. jw+RPW
-// of every plane, RPW + 1 rows of its buffer.  FULL: every lane's word is
-// inside the row (nx = 32 * LPR).
-
-// Block blk of the grid: row block blk % nyb, plane column blk / nyb.
-template <bool MC, bool FULL, int RPW, bool ALIGNED>
-__device__ __forceinline__ void count_tma_block(const float* __restrict__ vol, const Grid& g, float iso, int KC,
-                                                int nyb, int blk, uint4* __restrict__ rowcnt,
-                                                uint2* __restrict__ trims, uint32_t* __restrict__ mccnt,
-                                                uint32_t* __restrict__ bits_out,
-                                                unsigned long long* __restrict__ status)
-{
-    constexpr int LPR = 32 / RPW, NBUF = RPW + 1;
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ uint64_t s_bar[kCountRows];
-    const int jb = blk % nyb, kc = blk / nyb;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane / LPR, lw = lane % LPR;
-    const int jw = jb * kCountRows * RPW + RPW * warp;
-    if (jw >= g.ny) return;  // all the warp's rows past the grid
-    float* buf = reinterpret_cast<float*>(s_raw) + (size_t)warp * count_buffer_floats(g.nx, RPW, ALIGNED);
-    uint64_t* bar = &s_bar[warp];
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    const int j = jw + h;
-    const bool row_ok = j < g.ny;
-    const int kb = g.kr + kc * KC, ke = min(kb + KC, g.ke);
-    if (kb >= ke) {  // a block past the grid's last plane column: nothing to copy (no launch makes one today)
-        return;
-    }
-    const bool hasY = row_ok && j < g.ny - 1;
-    const int nq = g.nx >> 2;
-    const int nrows = min(NBUF, g.ny - jw);
-    const unsigned bytes = (unsigned)(nrows * g.nx * 4);
-    int lead = 0;      // points of the buffer before the warp's first row (ALIGNED false)
-    int tail_at = -1;  // this lane's place in the buffer for one of the rows' last points, or -1
-    float tail_v = 0.f;
-
-    // plane p -> buffer (lane 0 issues the copy); earlier reads of the buffer
-    // are ordered before the engine's writes by the caller's __syncwarp and
-    // the fence
-    auto issue = [&](int p) {
-        const long long s0 = ((long long)(p - g.kd) * g.ny + jw) * g.nx;
-        if (ALIGNED) {
-            if (lane == 0) {
-                fence_proxy_async();
-                mbar_arrive_expect_tx(bar, bytes);
-                bulk_copy_g2s(buf, vol + s0, bytes, bar);
-            }
-        } else {  // [a0, e0) by the engine, [max(e0, s0), e) by plain loads; all inside the volume
-            const long long a0 = s0 & ~3ll, e = s0 + (long long)nrows * g.nx, e0 = e & ~3ll;
-            const unsigned nb = e0 > a0 ? (unsigned)((e0 - a0) * 4) : 0u;
-            lead = (int)(s0 - a0);
-            if (lane == 0) {
-                fence_proxy_async();
-                mbar_arrive_expect_tx(bar, nb);
-                if (nb) bulk_copy_g2s(buf, vol + a0, nb, bar);
-            }
-            // loaded now, stored by take(): the warp does not wait here for the load
-            const long long lo = e0 > s0 ? e0 : s0;
-            tail_at = lane < (int)(e - lo) ? (int)(lo - a0) + lane : -1;
-            if (tail_at >= 0) tail_v = __ldg(vol + lo + lane);
-        }
-    };
-    unsigned phase = 0;
-    // words of rows A = buffer row h and B = buffer row h+1 of the plane in the buffer
-    auto take = [&](uint32_t& wa, uint32_t& wb) -> bool {
-        if (!ALIGNED && tail_at >= 0) buf[tail_at] = tail_v;
-        __syncwarp();  // the plain loads of the buffer's last points are visible
-        const bool done = mbar_wait(bar, phase);
-        if (!__all_sync(0xffffffffu, done)) return false;
-        phase ^= 1u;
-        if (ALIGNED) {
-            wa = row_ok ? row_word<FULL>(buf + h * g.nx, nq, lw, lane & 7, iso) : 0u;
-            wb = hasY ? row_word<FULL>(buf + (h + 1) * g.nx, nq, lw, lane & 7, iso) : 0u;
-        } else {
-            // every lane builds both words (the shuffles); rows past the grid read stale buffer rows
-            wa = row_word_shift(buf, lead + h * g.nx, g.nx, lw, lane & 7, lw == LPR - 1, iso);
-            wb = row_word_shift(buf, lead + (h + 1) * g.nx, g.nx, lw, lane & 7, lw == LPR - 1, iso);
-            wa = row_ok ? wa : 0u;
-            wb = hasY ? wb : 0u;
-            // the plain stores of the last points (lanes 0-2) may lie where the next copies write:
-            // each writer orders them before the async proxy, not only the lane that issues the copy
-            fence_proxy_async();
-        }
-        __syncwarp();  // every lane has read the buffer before it is refilled
-        return true;
-    };
-    // per-row totals: rows 2p, 2p+1 of the warp in the two 16-bit halves of reduction p (one row per warp:
-    // the warp's sum)
-    auto row_sum = [&](uint32_t v) -> uint32_t {
-        if (RPW == 1) return __reduce_add_sync(0xffffffffu, v);
-        const int sh = 16 * (h & 1);
-        uint32_t mine = 0u;
-#pragma unroll
-        for (int p = 0; p < RPW / 2; ++p) {
-            const uint32_t s = __reduce_add_sync(0xffffffffu, (h >> 1) == p ? v << sh : 0u);
-            if ((h >> 1) == p) mine = s;
-        }
-        return (mine >> sh) & 0xffffu;
-    };
-
-    uint32_t A = 0, B = 0, Cw = 0, Dw = 0;
-    bool ok = true;
-    issue(kb);
-    ok = take(A, B);
-    if (ok && kb + 1 < g.nz) issue(kb + 1);
-    for (int k = kb; ok && k < ke; ++k) {
-        const bool hasZ = k + 1 < g.nz;
-        Cw = Dw = 0u;
-        if (hasZ) {  // plane k+1 was issued one step earlier
-            if (!(ok = take(Cw, Dw))) break;
-            if (k + 2 < g.nz && k + 1 < ke) issue(k + 2);
-        }
-        RowCounts rc;
-        RowWords rw;
-        rw.a = A;
-        rw.b = B;
-        rw.c = Cw;
-        rw.d = Dw;
-        const uint32_t an = __shfl_down_sync(0xffffffffu, rw.a, 1, LPR);
-        const uint32_t bn = __shfl_down_sync(0xffffffffu, rw.b, 1, LPR);
-        const uint32_t cn = __shfl_down_sync(0xffffffffu, rw.c, 1, LPR);
-        const uint32_t dn = __shfl_down_sync(0xffffffffu, rw.d, 1, LPR);
-        const bool nxt = lw < LPR - 1;
-        rw.ash = (rw.a >> 1) | ((nxt ? an : 0u) << 31);
-        rw.bsh = (rw.b >> 1) | ((nxt ? bn : 0u) << 31);
-        rw.csh = (rw.c >> 1) | ((nxt ? cn : 0u) << 31);
-        rw.dsh = (rw.d >> 1) | ((nxt ? dn : 0u) << 31);
-        if (row_ok) count_word<MC>(rw, lw, g, j, k, hasY, hasZ, trims != nullptr, rc);
-        const long long r = (long long)(k - g.kr) * g.ny + j;
-        if (row_ok && lw < g.W) bits_out[r * g.W + lw] = rw.a;
-        const uint32_t sx = row_sum(rc.xc), sy = row_sum(rc.yc), sz = row_sum(rc.zc), st = row_sum(rc.tc);
-        const uint32_t sm = MC ? row_sum(rc.mc) : 0u;
-        uint32_t first = 0u, last = 0u;
-        if (trims) {  // each row's own minimum and maximum, the other rows contributing the identity
-#pragma unroll
-            for (int q = 0; q < RPW; ++q) {
-                const uint32_t f = __reduce_min_sync(0xffffffffu, h == q ? rc.first : 0xffffffffu);
-                const uint32_t x = __reduce_max_sync(0xffffffffu, h == q ? rc.last : 0u);
-                if (h == q) {
-                    first = f;
-                    last = x;
-                }
-            }
-        }
-        if (row_ok && lw == 0) {
-            rowcnt[r] = make_uint4(sx, sy, sz, st);
-            if (trims) trims[r] = make_uint2(first == 0xffffffffu ? (uint32_t)g.nx : first, last);
-            if (MC) mccnt[r] = sm;
-        }
-        A = Cw;
-        B = Dw;
-    }
-    if (!ok) {  // a copy did not complete in time: report it, and let the copy land before the CTA ends
-        if (lane == 0) atomicOr(status, kStatusTimeout);
-        mbar_wait(bar, phase);
-    }
-}
-
-template <bool MC, bool FULL, int RPW, bool ALIGNED>
-__global__ void __launch_bounds__(kThreads, 4) k_count_tma(const float* __restrict__ vol, Grid g, float iso, int KC,
-                                                        int nyb, uint4* __restrict__ rowcnt,
-                                                        uint2* __restrict__ trims, uint32_t* __restrict__ mccnt,
-                                                        uint32_t* __restrict__ bits_out,
-                                                        unsigned long long* __restrict__ status)
-{
-    count_tma_block<MC, FULL, RPW, ALIGNED>(vol, g, iso, KC, nyb, (int)blockIdx.x, rowcnt, trims, mccnt, bits_out,
-                                            status);
-}
-
-// The Flying Edges count blocks of a list of requests (batch_kernels.cuh), one launch.
-template <bool FULL, int RPW, bool ALIGNED>
-__global__ void __launch_bounds__(kThreads, 4) k_count_tma_batch(const BatchReq* __restrict__ reqs,
-                                                              const int* __restrict__ list,
-                                                              const unsigned* __restrict__ first, int m)
-{
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ uint64_t s_bar[kCountWarps];
+    const int warp = threadIdx.x >> 5;
     const int q = batch_find(first, m, blockIdx.x);
     const BatchReq* d = reqs + __ldg(&list[q]);
     const Grid g = d->g;
-    count_tma_block<false, FULL, RPW, ALIGNED>(d->vol, g, d->iso, d->count_KC, d->count_nyb,
-                                               (int)(blockIdx.x - __ldg(&first[q])), d->rowcnt, nullptr, nullptr,
-                                               d->bits, d->totals + 3);
+    const unsigned item = (blockIdx.x - __ldg(&first[q])) * kCountWarps + warp;
+    const FloatSamples<ALIGNED> smp(d->below);
+    count_rows_item<FloatSamples<ALIGNED>, false, kBatchCountRows>(
+        d->vol, g, smp, d->count_KC, d->count_groups, item, s_raw + (size_t)warp * stage_bytes,
+        s_bar + warp, d->rowcnt, nullptr, nullptr, d->bits, d->totals + 3);
 }
 
 // Word c*32 + lane of a row and, uniform over the warp, word c*32 + 32 (the
@@ -843,7 +639,32 @@ CountPlan count_plan(const Grid& g, int nsm)
     if (p.KC < 1) p.KC = 1;
     p.nkc = (nzw + p.KC - 1) / p.KC;
     p.nseg = (int)((g.R + kSeg - 1) / kSeg);
+    p.nsm = nsm;
     return p;
+}
+
+CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned, bool trims)
+{
+    CountRows r;
+    const int nzw = g.ke - g.kr;  // planes of the window
+    auto resident = [&](int S) {  // warps of one wave with S rows per lane
+        r.S = S;
+        r.stage = count_stage_bytes(g.nx, g.W, S, sample_bytes, aligned);
+        r.groups = (g.ny + (32 / g.W) * S - 1) / ((32 / g.W) * S);
+        const long long per_sm = (227ll * 1024) / (kCountWarps * (long long)r.stage + 1024);
+        return (long long)nsm * kCountWarps * std::max(1ll, std::min(8ll, per_sm));
+    };
+    // Rows of 17-32 words, one per warp at a time: four per lane where that leaves every warp of a wave at least 8
+    // planes (768^3: 302 us against 312 with two and 395 with one).  Else two, which is the best or within 1% of it
+    // from 256^3 (20.2 us, with four 21.8) to 512^3 (103.5, with four 105), and one where a wave's half has less
+    // than a plane each (64^3: 10.0 us against 11.9 with two).
+    long long warps = resident(trims ? 1 : (g.W > 16 ? 4 : 2));
+    if (r.S == 4 && (long long)r.groups * nzw < 8 * warps) warps = resident(2);
+    if (r.S == 2 && 2ll * r.groups * nzw < warps) warps = resident(1);
+    const long long cols = std::max(1ll, warps / r.groups);  // one wave
+    r.KC = (int)std::max(1ll, (nzw + cols - 1) / cols);
+    r.items = (unsigned)((long long)r.groups * ((nzw + r.KC - 1) / r.KC));
+    return r;
 }
 
 template <bool MC>
@@ -851,63 +672,36 @@ static void count_launch(const CountPlan& p, const float* vol, const Grid& g, fl
                          FeBuffers& b, cudaStream_t s)
 {
     const unsigned blocks = (unsigned)(p.nyb * p.nkc);
-    const bool vec4 = g.W <= 64 && (g.nx % 4 == 0) && ((reinterpret_cast<uintptr_t>(vol) & 15) == 0);
-    uint2* trims = p.trims ? b.trims : nullptr;  // the kernels skip the trims when null
     const bool base16 = (reinterpret_cast<uintptr_t>(vol) & 15) == 0;
-    if (base16 && g.W <= 32) {  // 8 rows per warp up to 4 words, 4 up to 8, 2 up to 16, else 1; planes via TMA
-        const int rpw = g.W <= 4 ? 8 : (g.W <= 8 ? 4 : (g.W <= 16 ? 2 : 1));
+    const bool vec4 = g.W <= 64 && (g.nx % 4 == 0) && base16;
+    uint2* trims = p.trims ? b.trims : nullptr;  // the kernels skip the trims when null
+    if (base16 && g.W <= 32) {
         const bool aligned = g.nx % 4 == 0;
-        const int rows = kCountRows * rpw;
-        const int nyb2 = (g.ny + rows - 1) / rows;
-        const unsigned blocks2 = (unsigned)(nyb2 * p.nkc);
-        const int nq = g.nx >> 2;
-        const size_t smem = (size_t)kCountRows * count_buffer_floats(g.nx, rpw, aligned) * sizeof(float);
-#define ISO_TMA(FULL, RPW, AL)                                                                                 \
-    {                                                                                                          \
-        auto kern = k_count_tma<MC, FULL, RPW, AL>;                                                           \
-        allow_smem(kern, smem);                                                                                \
-        kern<<<blocks2, kThreads, smem, s>>>(vol, g, iso, p.KC, nyb2, b.rowcnt, trims, b.mccnt, b.bits,         \
-                                             b.totals + 3);                                                    \
+        const CountRows r = count_rows_plan(g, p.nsm, 4, aligned, p.trims);
+        const size_t smem = (size_t)kCountWarps * r.stage;
+        const unsigned nb = (r.items + kCountWarps - 1) / kCountWarps;
+        auto kern = r.S == 4 ? (aligned ? k_count_rows<MC, 4, true> : k_count_rows<MC, 4, false>)
+                  : r.S == 2 ? (aligned ? k_count_rows<MC, 2, true> : k_count_rows<MC, 2, false>)
+                             : (aligned ? k_count_rows<MC, 1, true> : k_count_rows<MC, 1, false>);
+        allow_smem(kern, smem);
+        kern<<<nb, kCountThreads, smem, s>>>(vol, g, count_below(iso), r.KC, r.groups, r.items, r.stage, b.rowcnt,
+                                             trims, b.mccnt, b.bits, b.totals + 3);
+        return;
     }
-        if (!aligned) {
-            if (rpw == 8) ISO_TMA(false, 8, false)
-            else if (rpw == 4) ISO_TMA(false, 4, false)
-            else if (rpw == 2) ISO_TMA(false, 2, false)
-            else ISO_TMA(false, 1, false)
-        } else if (rpw == 1) {
-            if (nq == 256) ISO_TMA(true, 1, true)
-            else ISO_TMA(false, 1, true)
-        } else if (rpw == 8) {
-            if (nq == 32) ISO_TMA(true, 8, true)
-            else ISO_TMA(false, 8, true)
-        } else if (rpw == 4) {
-            if (nq == 64) ISO_TMA(true, 4, true)
-            else ISO_TMA(false, 4, true)
-        } else {
-            if (nq == 128) ISO_TMA(true, 2, true)
-            else ISO_TMA(false, 2, true)
-        }
-#undef ISO_TMA
+    if (g.W > 64) {
+        k_count_wide<MC><<<blocks, kThreads, 0, s>>>(vol, g, iso, p.KC, p.nyb, cases, b.rowcnt, trims, b.mccnt,
+                                                     b.bits);
         return;
     }
 #define ISO_COUNT(VEC, UU, NWW)                                                                                \
     k_count_warps<MC, VEC, UU, NWW><<<blocks, kThreads, 0, s>>>(vol, g, iso, p.KC, p.nyb, cases, b.rowcnt,     \
                                                                 trims, b.mccnt, b.bits)
-    if (vec4) {
-        switch (p.vec_u) {
-            case 1: ISO_COUNT(true, 1, 1); break;
-            case 2: ISO_COUNT(true, 2, 1); break;
-            case 4: ISO_COUNT(true, 4, 1); break;
-            case 8: ISO_COUNT(true, 8, 1); break;
-            default: ISO_COUNT(true, 16, 2); break;
-        }
+    if (vec4) {  // rows of 33-64 words; the shorter ones ran above
+        ISO_COUNT(true, 16, 2);
     } else if (g.W <= 32) {
         ISO_COUNT(false, 1, 1);
-    } else if (g.W <= 64) {
-        ISO_COUNT(false, 1, 2);
     } else {
-        k_count_wide<MC><<<blocks, kThreads, 0, s>>>(vol, g, iso, p.KC, p.nyb, cases, b.rowcnt, trims, b.mccnt,
-                                                     b.bits);
+        ISO_COUNT(false, 1, 2);
     }
 #undef ISO_COUNT
 }
@@ -920,44 +714,25 @@ void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* 
     else count_launch<false>(p, vol, g, iso, cases, b, s);
 }
 
-CountVariant count_variant(const Grid& g)
+BatchCount batch_count(const Grid& g, int planes)
 {
-    CountVariant v;
-    v.rpw = g.W <= 4 ? 8 : (g.W <= 8 ? 4 : 2);
-    v.aligned = g.nx % 4 == 0;
-    v.full = v.aligned && (g.nx >> 2) == 256 / v.rpw;  // nq = 32 * LPR / 4 points in quads
-    return v;
+    BatchCount c;
+    const int G = (32 / g.W) * kBatchCountRows;
+    c.aligned = g.nx % 4 == 0;
+    c.stage = count_stage_bytes(g.nx, g.W, kBatchCountRows, 4, c.aligned);
+    c.groups = (g.ny + G - 1) / G;
+    c.KC = std::min(planes, g.nz);
+    c.blocks = ((long long)c.groups * ((g.nz + c.KC - 1) / c.KC) + kCountWarps - 1) / kCountWarps;
+    return c;
 }
 
-size_t count_batch_smem(const Grid& g, const CountVariant& v)
+void launch_count_batch(bool aligned, const BatchReq* reqs, const int* list, const unsigned* first, int m,
+                        unsigned blocks, int stage, cudaStream_t s)
 {
-    return (size_t)kCountRows * count_buffer_floats(g.nx, v.rpw, v.aligned) * sizeof(float);
-}
-
-void launch_count_batch(const CountVariant& v, const BatchReq* reqs, const int* list, const unsigned* first, int m,
-                        unsigned blocks, size_t smem, cudaStream_t s)
-{
-#define ISO_TMA_BATCH(FULL, RPW, AL)                                                                           \
-    {                                                                                                          \
-        auto kern = k_count_tma_batch<FULL, RPW, AL>;                                                         \
-        allow_smem(kern, smem);                                                                                \
-        kern<<<blocks, kThreads, smem, s>>>(reqs, list, first, m);                                             \
-    }
-    if (!v.aligned) {
-        if (v.rpw == 8) ISO_TMA_BATCH(false, 8, false)
-        else if (v.rpw == 4) ISO_TMA_BATCH(false, 4, false)
-        else ISO_TMA_BATCH(false, 2, false)
-    } else if (v.rpw == 8) {
-        if (v.full) ISO_TMA_BATCH(true, 8, true)
-        else ISO_TMA_BATCH(false, 8, true)
-    } else if (v.rpw == 4) {
-        if (v.full) ISO_TMA_BATCH(true, 4, true)
-        else ISO_TMA_BATCH(false, 4, true)
-    } else {
-        if (v.full) ISO_TMA_BATCH(true, 2, true)
-        else ISO_TMA_BATCH(false, 2, true)
-    }
-#undef ISO_TMA_BATCH
+    const size_t smem = (size_t)kCountWarps * stage;
+    auto kern = aligned ? k_count_rows_batch<true> : k_count_rows_batch<false>;
+    allow_smem(kern, smem);
+    kern<<<blocks, kCountThreads, smem, s>>>(reqs, list, first, m, stage);
 }
 
 void launch_scan_batch(const BatchReq* reqs, const int* list, const unsigned* first, int m, unsigned blocks,

@@ -32,7 +32,15 @@ struct CountPlan {
     int J = 8, nyb = 1, KC = 1, nkc = 1;
     int vec_u = 1;  // float4 loads per lane for one row (rows up to 64 words)
     int nseg = 1;
+    int nsm = 0;      // SMs of the device the plan is for
     bool trims = false;  // write the row trims (only the pass-by-pass interface reads them)
+};
+
+// Work split of the count pass over rows of up to 32 words (count_rows.cuh):
+// items of (32 / W) * S grid rows and KC planes, one warp each.
+struct CountRows {
+    int S = 1, stage = 0, groups = 1, KC = 1;
+    unsigned items = 0;
 };
 
 // Work split of the warp-per-row generate kernels: blocks of J = 8 rows,
@@ -73,6 +81,7 @@ inline void allow_smem(K kern, size_t dyn)
         cur = dyn;
 }
 CountPlan count_plan(const Grid& g, int nsm);
+CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned, bool trims);
 GenPlan gen_plan(const Grid& g, int nsm);
 void gen_split(GenPlan& p, int nsm);  // columns over [p.kbeg, p.kend)
 
