@@ -53,7 +53,7 @@ void replan(iso_ctx* ctx, std::vector<BatchItem>& items, const std::vector<int>&
 // ---------------------------------------------------------------------------
 struct FusedGroup {
     bool aligned = false;      // count: rows a multiple of 4 points
-    int rpw = 0, index_bytes = 4;
+    int index_bytes = 4;
     std::vector<int> members;  // descriptor indices
     unsigned total = 0;        // blocks (count, scan) or work items (generate)
     size_t list_at = 0, first_at = 0;
@@ -93,8 +93,8 @@ bool fusable(const iso_ctx* ctx, const iso_request& r, const BatchItem& it)
 // Work split of the fused launches: count blocks of at least kc planes, generate items for about ipw per warp
 // of one wave (the autotuner's candidates; 0: the defaults).
 constexpr int kFusedKC[] = {8, 16, 32};
-constexpr int kFusedIPW[] = {16, 32, 64};
-constexpr int kFusedKCDefault = 16, kFusedIPWDefault = 32;
+constexpr int kFusedIPW[] = {8, 16, 32};
+constexpr int kFusedKCDefault = 16, kFusedIPWDefault = 16;
 
 FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, std::vector<BatchItem>& items,
                      const std::vector<int>& fz, const iso::PackedOut* pk = nullptr, int kc_min = 0, int ipw = 0)
@@ -136,19 +136,17 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
         cg.stage = std::max(cg.stage, bc.stage);
         f.all.members.push_back(d);
         if (extract) {
-            const int rpw = iso::gen_rows_per_warp(g.W);
             const int ib = out ? out[r].index_bytes : pk->index_bytes;
-            const int gk = rpw | (ib << 8);
+            const int gk = ib;
             if (!gkey.count(gk)) {
                 gkey[gk] = (int)f.gen.size();
                 f.gen.emplace_back();
-                f.gen.back().rpw = rpw;
                 f.gen.back().index_bytes = ib;
             }
             FusedGroup& gg = f.gen[gkey[gk]];
             gg.members.push_back(d);
-            gg.ws_bytes = std::max(gg.ws_bytes, (int)iso::gen_batch_ws_bytes(g.W, rpw));
-            x.gen_ngroups = (g.ny + rpw - 1) / rpw;
+            gg.ws_bytes = std::max(gg.ws_bytes, iso::gen_batch_ws_bytes(g.W));
+            x.gen_ngroups = (g.ny + iso::gen_batch_rows(g.W) - 1) / iso::gen_batch_rows(g.W);
             gen_planes += (long long)x.gen_ngroups * g.nz;
         }
     }
@@ -227,6 +225,7 @@ void fill_fused(iso_ctx* ctx, const FusedPlan& f, const iso_mesh* out, const std
         carve(base + f.scratch_at[d], it.g, it.pl.cp, b);
         iso::BatchReq x = f.proto[d];
         x.rowcnt = b.rowcnt;
+        x.row4 = b.row4;
         x.bits = b.bits;
         x.starts = b.starts;
         x.part = b.part;
@@ -292,7 +291,7 @@ void enqueue_fused(iso_ctx* ctx, const FusedPlan& f, bool extract, cudaStream_t 
         iso::launch_vfirst_batch(D, L(f.all), nf, vfirst, s);
     fan_out(ctx, f.gen, s, [&](size_t q, cudaStream_t st) {
         const FusedGroup& g = f.gen[q];
-        iso::launch_gen_batch(g.rpw, g.index_bytes, D, L(g), F(g), (int)g.members.size(), g.total, ctx->d_cases,
+        iso::launch_gen_batch(g.index_bytes, D, L(g), F(g), (int)g.members.size(), g.total, ctx->d_cases,
                               work + q, g.ws_bytes, ctx->reverse, ctx->nsm, st);
     });
     iso::launch_vertices_batch(D, L(f.all), vfirst, nf, ctx->nsm, s);
@@ -434,7 +433,6 @@ std::vector<unsigned char> batch_key(const iso_ctx* ctx, int lanes, int share, c
             put(&g.total, sizeof g.total);
             put(&g.stage, sizeof g.stage);
             put(&g.ws_bytes, sizeof g.ws_bytes);
-            put(&g.rpw, sizeof g.rpw);
             put(&g.index_bytes, sizeof g.index_bytes);
             const int al = g.aligned ? 1 : 0;
             put(&al, sizeof al);

@@ -18,6 +18,7 @@ namespace iso {
 struct BatchReq {
     const float* vol;
     uint4* rowcnt;
+    uint4* row4;
     uint32_t* bits;
     unsigned long long* starts;
     unsigned long long* part;
@@ -64,8 +65,8 @@ struct BatchCount {
     long long blocks;
 };
 BatchCount batch_count(const Grid& g, int planes);
-// Rows per warp of the generate pass (rows of up to 16 words).
-inline int gen_rows_per_warp(int W) { return W <= 4 ? 8 : (W <= 8 ? 4 : 2); }
+// Rows of a generate item.
+int gen_batch_rows(int W);
 
 void launch_count_batch(bool aligned, const BatchReq* reqs, const int* list, const unsigned* first, int m,
                         unsigned blocks, int stage, cudaStream_t s);
@@ -78,12 +79,12 @@ void launch_vfirst_batch(const BatchReq* reqs, const int* list, int m, unsigned 
 // placed requests.
 void launch_place_batch(BatchReq* reqs, const int* list, int m, const PackedOut& out, unsigned long long* vfirst,
                         cudaStream_t s);
-void launch_gen_batch(int rpw, int index_bytes, const BatchReq* reqs, const int* list, const unsigned* first, int m,
+void launch_gen_batch(int index_bytes, const BatchReq* reqs, const int* list, const unsigned* first, int m,
                       unsigned nitems, const CaseTables* cases, unsigned* work, int ws_bytes, int reverse, int nsm,
                       cudaStream_t s);
 void launch_vertices_batch(const BatchReq* reqs, const int* list, const unsigned long long* vfirst, int m, int nsm,
                            cudaStream_t s);
 // Shared memory per warp of the generate kernel for rows of W words.
-size_t gen_batch_ws_bytes(int W, int rpw);
+int gen_batch_ws_bytes(int W);
 
 }  // namespace iso

@@ -119,7 +119,6 @@ iso_status slab_generate(iso_ctx* ctx, iso_algorithm algo, const float* volume, 
         gp.kbeg = (int)k0;
         gp.kend = (int)k1;
         gp.kemit = (int)k0;
-        iso::gen_split(gp, ctx->nsm);
         if (i4)
             iso::launch_fe_gen_warps<uint32_t>(volume, g, isoval, ctx->d_cases, b, pl.cp, gp, big, big, out->points,
                                                out->normals, static_cast<uint32_t*>(out->tris), ctx->reverse, s);
@@ -133,14 +132,12 @@ iso_status slab_generate(iso_ctx* ctx, iso_algorithm algo, const float* volume, 
         gp.kbeg = g.kr;  // cell row k0-1 maps the edges it owns on plane k0
         gp.kend = (int)k1;
         gp.kemit = (int)k0;
-        iso::gen_split(gp, ctx->nsm);
         iso::launch_mc_gen_warps(volume, g, isoval, ctx->d_cases, b, pl.cp, gp, big, big, out->points, out->normals,
                                  ctx->reverse, s);
         pm.mark(ISO_PASS_MC_VERTICES);
         if (iso::launch_mc_vertices(volume, g, isoval, b, gp, big, big, out->points, out->normals, s))
             pm.mark(ISO_PASS_VERTICES);
         gp.kbeg = (int)k0;
-        iso::gen_split(gp, ctx->nsm);
         if (i4)
             iso::launch_mc_tri_warps<uint32_t>(g, ctx->d_cases, b, pl.cp, gp, big, big,
                                                static_cast<uint32_t*>(out->tris), s);

@@ -132,6 +132,26 @@ inline void build_case_tables(CaseTables& t)
         }
         t.order[c] = order | ((uint64_t)n << 60);
     }
+    for (int m = 0; m < 256; ++m) {
+        const int c = (m & 0x33) | ((m & 0x44) << 1) | ((m & 0x88) >> 1);
+        t.order2[m] = t.order[c];
+        t.cut2[m] = t.cut[c];
+        t.nt2[m] = (uint8_t)iso_case_ntris(t.tris[c]);
+        for (int q = 0; q < 5; ++q) {
+            uint32_t x = 0;
+            for (int v = 0; v < 3 && q < t.nt2[m]; ++v) {
+                const int e = iso_case_edge(t.tris[c], 3 * q + v);  // cube_edge_geometry's low point and axis
+                const int dx = (0xA22 >> e) & 1, dy = (0xC44 >> e) & 1, dz = (0x0F0 >> e) & 1;
+                const int axis = e >= 8 ? 2 : (e & 1);
+                x |= (uint32_t)(16 * axis + 48 * dy + 8 * dz + dx) << (8 * v);
+            }
+            t.corner[5 * m + q] = x;
+        }
+        uint32_t places = 0;
+        for (int b = 0, n = 0; b < 8; ++b)
+            if ((m >> b) & 1) places |= (uint32_t)b << (4 * n++);
+        t.nth[m] = places;
+    }
 }
 
 inline bool valid_algo(iso_algorithm a)
@@ -165,7 +185,7 @@ inline bool empty_grid(const Grid& g) { return g.nx < 2 || g.ny < 2 || g.nz < 2;
 inline size_t scratch_size(const Grid& g, const iso::CountPlan& cp)
 {
     const size_t R = (size_t)g.R;
-    return align256(R * 16) + align256(R * 8) + align256(R * 4) + align256(4 * R * 8) +
+    return 2 * align256(R * 16) + align256(R * 8) + align256(R * 4) + align256(4 * R * 8) +
            align256(4 * (size_t)cp.nseg * 8) + align256(8 * 8) + align256(R * (size_t)g.W * 4);
 }
 
@@ -174,6 +194,7 @@ inline void carve(void* base, const Grid& g, const iso::CountPlan& cp, FeBuffers
     const size_t R = (size_t)g.R;
     char* p = static_cast<char*>(base);
     b.rowcnt = reinterpret_cast<uint4*>(p); p += align256(R * 16);
+    b.row4 = reinterpret_cast<uint4*>(p); p += align256(R * 16);
     b.trims = reinterpret_cast<uint2*>(p); p += align256(R * 8);
     b.mccnt = reinterpret_cast<uint32_t*>(p); p += align256(R * 4);
     b.starts = reinterpret_cast<unsigned long long*>(p); p += align256(4 * R * 8);

@@ -386,7 +386,7 @@ template <int SM>
 __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcnt,
                                                  const uint32_t* __restrict__ mccnt, long long R,
                                                  const unsigned long long* __restrict__ part, int nseg,
-                                                 unsigned long long* __restrict__ starts,
+                                                 unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
                                                  unsigned long long* __restrict__ totals, int blk)
 {
     constexpr int NC = ScanComps<SM>::n;
@@ -444,6 +444,10 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
 #pragma unroll
         for (int q = 0; q < kScanPer; ++q) {
             if (b + q < R) starts[a * R + b + q] = run;
+            if (SM != kScanDup && a == 0 && b + q < R) {  // the row's vertices are its x, its y, then its z cuts
+                const uint2 c = __ldg(reinterpret_cast<const uint2*>(rowcnt + b + q));
+                row4[b + q] = make_uint4((uint32_t)run, (uint32_t)run + c.x, (uint32_t)run + c.x + c.y, 0u);
+            }
             run += v[a][q];
         }
     }
@@ -454,9 +458,10 @@ __global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* __restrict
                                                          const uint32_t* __restrict__ mccnt, long long R,
                                                          const unsigned long long* __restrict__ part, int nseg,
                                                          unsigned long long* __restrict__ starts,
+                                                         uint4* __restrict__ row4,
                                                          unsigned long long* __restrict__ totals)
 {
-    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, totals, (int)blockIdx.x);
+    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, row4, totals, (int)blockIdx.x);
 }
 
 // The Flying Edges scans of a list of requests, one launch per phase: block x is segment
@@ -480,7 +485,8 @@ __global__ void __launch_bounds__(kThreads) k_scan_final_batch(const BatchReq* _
     const BatchReq* d = reqs + __ldg(&list[q]);
     const int blk = (int)(blockIdx.x - __ldg(&first[q]));
     if (blk >= d->nseg) return;
-    scan_final_block<kScanFE>(d->rowcnt, nullptr, d->g.R, d->part, d->nseg, d->starts, d->totals, blk);
+    scan_final_block<kScanFE>(d->rowcnt, nullptr, d->g.R, d->part, d->nseg, d->starts, d->row4,
+                              d->totals, blk);
 }
 
 // vfirst[q] = the vertices of requests list[0 .. q-1] whose meshes hold their counts (one CTA of 1024 threads,
@@ -757,7 +763,7 @@ void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cuda
 {
 #define ISO_SCAN(SM)                                                                                            \
     k_scan_partial<SM><<<p.nseg, kThreads, 0, s>>>(b.rowcnt, b.mccnt, g.R, b.part, p.nseg);                      \
-    k_scan_final<SM><<<p.nseg, kThreads, 0, s>>>(b.rowcnt, b.mccnt, g.R, b.part, p.nseg, b.starts, b.totals)
+    k_scan_final<SM><<<p.nseg, kThreads, 0, s>>>(b.rowcnt, b.mccnt, g.R, b.part, p.nseg, b.starts, b.row4, b.totals)
     if (mode == kScanMC) {
         ISO_SCAN(kScanMC);
     } else if (mode == kScanDup) {

@@ -1,51 +1,24 @@
-// Flying Edges pass 4 (two or four rows per warp, gen_pairs.cuh, for rows of up to 16
-// words; else one row per warp, gen_warps.cuh) and the plan of the
-// warp-per-row kernels.
+// Flying Edges pass 4 (gen_cells.cuh), its vertices from the records
+// (vertices.cuh), and the plan of the generate kernels.
 #include "../../include/miniiso.h"
-#include "gen_pairs.cuh"
-#include "gen_warps.cuh"
+#include "gen_cells.cuh"
 
 namespace iso {
 
-// Warp-per-row kernels take rows of up to 32 words (1024 points) whose cell
-// rows number their vertices in 32 bits relative to the row's first one;
-// wider grids use the row-wise kernels.
-// Columns of KC planes over [kbeg, kend): about 4 waves of resident CTAs,
-// at least 4 planes per column.
-void gen_split(GenPlan& p, int nsm)
-{
-    p.nsm = nsm;
-    const int nzw = p.kend - p.kbeg;
-    const long long resident = (long long)nsm * kGenCtasPerSm;
-    int nkc = (int)((4 * resident + p.nyb - 1) / p.nyb);
-    if (nkc < 1) nkc = 1;
-    p.KC = (nzw + nkc - 1) / nkc;
-    if (p.KC < 4) p.KC = 4;
-    if (p.KC > nzw) p.KC = nzw;
-    if (p.KC < 1) p.KC = 1;
-    p.nkc = nzw > 0 ? (nzw + p.KC - 1) / p.KC : 0;
-}
-
+// The generate kernels take rows of up to 32 words (1024 points) whose warps
+// number their vertices in 32 bits relative to one row's first one; wider grids
+// use the row-wise kernels.
 GenPlan gen_plan(const Grid& g, int nsm)
 {
     GenPlan p;
-    p.J = kGenRows;
-    p.nyb = (g.ny + p.J - 1) / p.J;
-    p.smem = (size_t)kGenRows * gen_warp_scratch_bytes(g.W, kGenMC);
+    p.nsm = nsm;
     const bool rel32 = 6.0 * g.nx * g.ny < 4294967295.0;  // two planes of vertices
     // vertex records pack i < 2^10, j < 2^27, k < 2^22
     p.fits = g.W <= 32 && rel32 && g.ny < (1 << 27) && g.nz < (1 << 22);
     p.kbeg = g.kr;
     p.kend = g.ke;
     p.kemit = g.kr;
-    gen_split(p, nsm);
     return p;
-}
-
-// Grids whose pass 4 runs as k_gen_pairs + k_vertices.
-static bool fe_writes_records(const Grid& g, const GenPlan& p)
-{
-    return g.W <= 16 && p.nsm > 0;
 }
 
 template <typename IndexT>
@@ -53,17 +26,13 @@ void launch_fe_gen_warps(const float* vol, const Grid& g, float iso, const CaseT
                          const CountPlan& cp, const GenPlan& p, long long capV, long long capT, float* points,
                          float* normals, IndexT* tris, int reverse, cudaStream_t s)
 {
-    if (fe_writes_records(g, p))  // several rows per warp
-        launch_gen_pairs_impl<IndexT, kGenFE>(g, cases, b, cp, p, p.nsm, capV, capT, points, tris, reverse, s);
-    else
-        launch_gen_warps_impl<kGenFE, IndexT>(vol, g, iso, cases, b, cp, p, capV, capT, points, normals, tris,
-                                              reverse, s);
+    launch_gen_cells<IndexT, kGenFE>(g, cases, b, cp, p, capV, capT, points, tris, reverse, s);
 }
 
 bool launch_fe_vertices(const float* vol, const Grid& g, float iso, const FeBuffers& b, const GenPlan& p,
                         long long capV, long long capT, float* points, float* normals, cudaStream_t s)
 {
-    if (!fe_writes_records(g, p)) return false;
+    if (p.nsm <= 0) return false;
     launch_vertices_impl<false, 0>(vol, g, iso, b, p.kbeg, p.kend, p.nsm, capV, capT, points, normals, s);
     return true;
 }
@@ -72,7 +41,7 @@ bool launch_fe_vertices_narrow(const void* vol, int dtype, const Grid& g, float 
                                const GenPlan& p, long long capV, long long capT, float* points, float* normals,
                                cudaStream_t s)
 {
-    if (!fe_writes_records(g, p)) return false;
+    if (p.nsm <= 0) return false;
     switch (dtype) {
         case ISO_INT8:
             launch_vertices_impl<false, 0, int8_t>(static_cast<const int8_t*>(vol), g, iso, b, p.kbeg, p.kend, p.nsm,
@@ -140,32 +109,27 @@ __global__ void __launch_bounds__(kThreads, vertex_ctas_per_sm(false))
     }
 }
 
-size_t gen_batch_ws_bytes(int W, int rpw) { return gen_pair_scratch_bytes(W, rpw, kGenFE); }
+int gen_batch_ws_bytes(int W) { return gen_cells_scratch(W, 32 / W, kGenFE); }
 
-void launch_gen_batch(int rpw, int index_bytes, const BatchReq* reqs, const int* list, const unsigned* first, int m,
+int gen_batch_rows(int W) { return gen_held_rows(32 / W) - 1; }
+
+void launch_gen_batch(int index_bytes, const BatchReq* reqs, const int* list, const unsigned* first, int m,
                       unsigned nitems, const CaseTables* cases, unsigned* work, int ws_bytes, int reverse, int nsm,
                       cudaStream_t s)
 {
-    long long blocks = ((long long)nitems + kGenRows - 1) / kGenRows;
-    if (blocks > (long long)nsm * kGenPairCtasPerSm) blocks = (long long)nsm * kGenPairCtasPerSm;
+    const int warps = gen_cells_warps(ws_bytes, sizeof(GenCellTables<kGenFE>));
+    const long long blocks = std::min(((long long)nitems + warps - 1) / warps, 2ll * nsm);
     if (blocks < 1) return;
-    const size_t smem = (size_t)kGenRows * ws_bytes;
-#define ISO_GEN_BATCH(T, R)                                                                                    \
-    {                                                                                                          \
-        auto kern = k_gen_pairs_batch<T, R>;                                                                   \
-        allow_smem(kern, smem);                                                                                \
-        kern<<<(unsigned)blocks, kThreads, smem, s>>>(reqs, list, first, m, cases, work, ws_bytes, reverse);    \
-    }
+    const size_t smem = (size_t)warps * ws_bytes;
     if (index_bytes == 4) {
-        if (rpw == 8) ISO_GEN_BATCH(uint32_t, 8)
-        else if (rpw == 4) ISO_GEN_BATCH(uint32_t, 4)
-        else ISO_GEN_BATCH(uint32_t, 2)
+        allow_smem(k_gen_cells_batch<uint32_t>, smem);
+        k_gen_cells_batch<uint32_t><<<(unsigned)blocks, 32 * warps, smem, s>>>(reqs, list, first, m, cases, work,
+                                                                               ws_bytes, reverse);
     } else {
-        if (rpw == 8) ISO_GEN_BATCH(uint64_t, 8)
-        else if (rpw == 4) ISO_GEN_BATCH(uint64_t, 4)
-        else ISO_GEN_BATCH(uint64_t, 2)
+        allow_smem(k_gen_cells_batch<uint64_t>, smem);
+        k_gen_cells_batch<uint64_t><<<(unsigned)blocks, 32 * warps, smem, s>>>(reqs, list, first, m, cases, work,
+                                                                               ws_bytes, reverse);
     }
-#undef ISO_GEN_BATCH
 }
 
 void launch_vertices_batch(const BatchReq* reqs, const int* list, const unsigned long long* vfirst, int m, int nsm,

@@ -1,10 +1,9 @@
-// Marching Cubes pass 4 (the kernels of gen_pairs.cuh for rows of up to 16
-// words, else the warp-per-row kernels of gen_warps.cuh): vertex records
-// in owner order with the Flying Edges -> MC index map, the vertices from the
-// records (vertices.cuh), then the triangles with their corners mapped; and
-// the duplicate-free order in one pass.
+// Marching Cubes pass 4 (gen_cells.cuh): vertex records in owner order with the
+// Flying Edges -> MC index map, the vertices from the records (vertices.cuh),
+// and the triangles with their corners mapped; and the duplicate-free order in
+// one pass (gen_warps.cuh).
 #include "../../include/miniiso.h"
-#include "gen_pairs.cuh"
+#include "gen_cells.cuh"
 #include "gen_warps.cuh"
 #include "vertices.cuh"
 
@@ -14,11 +13,7 @@ void launch_mc_gen_warps(const float* vol, const Grid& g, float iso, const CaseT
                          const CountPlan& cp, const GenPlan& p, long long capV, long long capT, float* points,
                          float* normals, int reverse, cudaStream_t s)
 {
-    if (g.W <= 16 && p.nsm > 0)  // several rows per warp
-        launch_gen_pairs_impl<uint32_t, kGenMC>(g, cases, b, cp, p, p.nsm, capV, capT, points, nullptr, reverse, s);
-    else
-        launch_gen_warps_impl<kGenMC, uint32_t>(vol, g, iso, cases, b, cp, p, capV, capT, points, normals, nullptr,
-                                                reverse, s);
+    launch_gen_cells<uint32_t, kGenMC>(g, cases, b, cp, p, capV, capT, points, nullptr, reverse, s);
 }
 
 bool launch_mc_vertices(const float* vol, const Grid& g, float iso, const FeBuffers& b, const GenPlan& p,
@@ -63,18 +58,18 @@ bool launch_dup_vertices(const float* vol, const Grid& g, float iso, const FeBuf
     return true;
 }
 
-// Marching Cubes over rows of up to 16 words in two passes instead of
-// three: the owned vertices (records, FE -> MC map) and the triangles with
-// the corners' Flying Edges ids in one generate pass, then k_mc_remap
-// replaces every index by its MC id once the map is complete.
-bool mc_fused(const Grid& g, const GenPlan& p) { return g.W <= 16 && p.nsm > 0 && p.kemit == g.kr; }
+// Marching Cubes over whole windows in two passes instead of three: the owned
+// vertices (records, FE -> MC map) and the triangles with the corners' Flying
+// Edges ids in one generate pass, then k_mc_remap replaces every index by its MC
+// id once the map is complete.
+bool mc_fused(const Grid& g, const GenPlan& p) { return p.nsm > 0 && p.kemit == g.kr; }
 
 template <typename IndexT>
 void launch_mc_gen_tris(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                         const GenPlan& p, long long capV, long long capT, float* points, IndexT* tris, int reverse,
                         cudaStream_t s)
 {
-    launch_gen_pairs_impl<IndexT, kGenMCT>(g, cases, b, cp, p, p.nsm, capV, capT, points, tris, reverse, s);
+    launch_gen_cells<IndexT, kGenMCT>(g, cases, b, cp, p, capV, capT, points, tris, reverse, s);
 }
 
 // tris[i] = fe2mc[tris[i]] for the 3 T indices (T from the totals); nothing
@@ -169,11 +164,7 @@ template <typename IndexT>
 void launch_mc_tri_warps(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                          const GenPlan& p, long long capV, long long capT, IndexT* tris, cudaStream_t s)
 {
-    if (g.W <= 16 && p.nsm > 0)  // several rows per warp
-        launch_gen_pairs_impl<IndexT, kGenTri>(g, cases, b, cp, p, p.nsm, capV, capT, nullptr, tris, 0, s);
-    else
-        launch_gen_warps_impl<kGenTri, IndexT>(nullptr, g, 0.f, cases, b, cp, p, capV, capT, nullptr, nullptr, tris,
-                                               0, s);
+    launch_gen_cells<IndexT, kGenTri>(g, cases, b, cp, p, capV, capT, nullptr, tris, 0, s);
 }
 
 template <typename IndexT>
@@ -181,8 +172,7 @@ void launch_dup_gen_warps(const float* vol, const Grid& g, float iso, const Case
                           const CountPlan& cp, const GenPlan& p, long long capV, long long capT, float* points,
                           float* normals, IndexT* tris, int reverse, cudaStream_t s)
 {
-    launch_gen_warps_impl<kGenDup, IndexT>(vol, g, iso, cases, b, cp, p, capV, capT, points, normals, tris, reverse,
-                                           s);
+    launch_gen_dup<IndexT>(g, cases, b, cp, p, capV, capT, points, tris, reverse, s);
 }
 
 template void launch_dup_gen_warps<uint32_t>(const float*, const Grid&, float, const CaseTables*, const FeBuffers&,

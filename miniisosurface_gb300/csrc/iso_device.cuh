@@ -44,6 +44,14 @@ struct CaseTables {
     uint64_t order[256];   // cube edges in order of first appearance in the
                            // triangle list, packed like tris (count in 60..63)
     uint16_t cut[256];     // 12-bit mask of the cut cube edges of the case
+    // The same by the case number of gen_cells.cuh: bits 2 and 3, and 6 and 7,
+    // change places (the corners of rows B and D in x order).
+    uint32_t corner[256 * 5];  // per triangle: a byte per corner, its edge's place in the warp's table
+                               // (axis * 16 + next row * 48 + next plane * 8, bit 0: the edge at point i + 1)
+    uint32_t nth[256];     // of a byte: the places of its set bits, a nibble each
+    uint64_t order2[256];
+    uint16_t cut2[256];
+    uint8_t nt2[256];      // triangles of the case
 };
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }

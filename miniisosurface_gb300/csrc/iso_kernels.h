@@ -16,6 +16,7 @@ struct RowStarts;
 // launchers).  R = ny*nz grid rows, W = ceil(nx/32) words per row.
 struct FeBuffers {
     uint4* rowcnt = nullptr;               // R      x/y/z cuts, triangles
+    uint4* row4 = nullptr;                 // R      low 32 bits of the row's first x, y and z cut's ids (scan)
     uint2* trims = nullptr;                // R      xl, xr (pass 1 trims)
     uint32_t* mccnt = nullptr;             // R      MC vertices per cell row
     unsigned long long* starts = nullptr;  // 4*R    per row: first vertex, triangle, MC vertex (or y, z cuts)
@@ -43,16 +44,13 @@ struct CountRows {
     unsigned items = 0;
 };
 
-// Work split of the warp-per-row generate kernels: blocks of J = 8 rows,
-// columns of KC planes over planes [kbeg, kend).  For a slab: rows below
+// What the generate kernels cover: planes [kbeg, kend).  For a slab: rows below
 // kemit only map (MC), ids are shifted by add[] and stored at id - vbase
 // (vertices) and t - tbase (triangles).
 struct GenPlan {
-    int J = 8, nyb = 1, KC = 1, nkc = 1;
     int kbeg = 0, kend = 0, kemit = 0;
     unsigned long long vbase = 0, tbase = 0;
     unsigned long long add[4] = {0, 0, 0, 0};
-    size_t smem = 0;  // per-warp scratch of the CTA
     int nsm = 0;      // SMs of the device the plan is for
     bool fits = false;  // false: use the row-wise kernels
 };
@@ -83,7 +81,6 @@ inline void allow_smem(K kern, size_t dyn)
 CountPlan count_plan(const Grid& g, int nsm);
 CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned, bool trims);
 GenPlan gen_plan(const Grid& g, int nsm);
-void gen_split(GenPlan& p, int nsm);  // columns over [p.kbeg, p.kend)
 
 // passes 1-3
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
@@ -93,7 +90,7 @@ void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cuda
 // totals and the starts of rows rlo / rhi into out[0..8] (device-visible host memory)
 void launch_slab_readback(const FeBuffers& b, const Grid& g, long long rlo, long long rhi, bool has_lo, bool has_hi,
                           unsigned long long* out, cudaStream_t s);
-// Marching Cubes in two passes (rows of up to 16 words, whole windows): owned
+// Marching Cubes in two passes (rows of up to 32 words, whole windows): owned
 // vertices and FE-id triangles together, then the triangles' ids remapped
 bool mc_fused(const Grid& g, const GenPlan& p);
 template <typename IndexT>
@@ -113,9 +110,8 @@ void launch_grid_edges(const Grid& g, const CountPlan& p, const FeBuffers& b, in
 // Row-start accessor of a counted extraction.
 RowStarts row_starts(const Grid& g, const CountPlan& p, const FeBuffers& b);
 
-// pass 4, Flying Edges: rows of up to 16 words two per warp, writing vertex
-// records that launch_fe_vertices turns into vertices (it returns false, and
-// launches nothing, for the grids whose generate pass computes them itself)
+// pass 4, Flying Edges: triangles, and vertex records that launch_fe_vertices
+// turns into vertices (false: nothing launched, the plan cannot run it)
 template <typename IndexT>
 void launch_fe_gen_warps(const float* vol, const Grid& g, float iso, const CaseTables* cases, const FeBuffers& b,
                          const CountPlan& cp, const GenPlan& p, long long capV, long long capT, float* points,

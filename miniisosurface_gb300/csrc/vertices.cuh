@@ -1,5 +1,5 @@
 // Pass 4 vertex values from records (included by gen_warps_fe.cu through
-// gen_pairs.cuh and by gen_warps_mc.cu).
+// gen_cells.cuh, and by gen_warps_mc.cu).
 //
 // The generate kernels do not compute vertices: for every vertex they write a
 // record into the first 8 bytes of its own 12-byte slot of the points buffer,
