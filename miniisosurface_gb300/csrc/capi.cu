@@ -682,17 +682,17 @@ iso_status iso_count_device(iso_ctx* ctx, iso_algorithm algo, const float* volum
     iso_status st = ensure_scratch(ctx, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     PassMarks pm(ctx, s);
-    enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm);
+    enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm, ctx->h_totals);
     ISO_CUDA(ctx, cudaGetLastError());
-    ISO_CUDA(ctx, cudaMemcpyAsync(ctx->h_totals, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
     *n_points = (int64_t)ctx->h_totals[0];
     *n_tris = (int64_t)ctx->h_totals[1];
     return ISO_OK;
 }
 
-iso_status iso_extract_device_async(iso_ctx* ctx, iso_algorithm algo, const float* volume, const iso_grid* grid,
-                                    float isoval, iso_mesh* out, int64_t* result_host, void* stream)
+// sync: result_host is the context's own h_totals, which the scan writes itself, and the call is not captured.
+static iso_status extract_device(iso_ctx* ctx, iso_algorithm algo, const float* volume, const iso_grid* grid,
+                                 float isoval, iso_mesh* out, int64_t* result_host, void* stream, bool sync)
 {
     if (!ctx || !grid || !result_host) return ISO_ERR_INVALID_ARG;
     if (!valid_algo(algo)) return ISO_ERR_INVALID_ARG;
@@ -721,11 +721,19 @@ iso_status iso_extract_device_async(iso_ctx* ctx, iso_algorithm algo, const floa
     if (ctx->one_graph && !ctx->profiling) return extract_graph(ctx, algo, volume, g, grid, isoval, pl, b, out,
                                                                 result_host, s);
     PassMarks pm(ctx, s);
-    enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm);
+    enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm, sync ? ctx->h_totals : nullptr);
     enqueue_generate(ctx, algo, volume, g, isoval, pl, b, out, s, pm);
     ISO_CUDA(ctx, cudaGetLastError());
-    ISO_CUDA(ctx, cudaMemcpyAsync(result_host, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    if (!sync)
+        ISO_CUDA(ctx,
+                 cudaMemcpyAsync(result_host, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     return ISO_OK;
+}
+
+iso_status iso_extract_device_async(iso_ctx* ctx, iso_algorithm algo, const float* volume, const iso_grid* grid,
+                                    float isoval, iso_mesh* out, int64_t* result_host, void* stream)
+{
+    return extract_device(ctx, algo, volume, grid, isoval, out, result_host, stream, false);
 }
 
 iso_status iso_extract_device(iso_ctx* ctx, iso_algorithm algo, const float* volume, const iso_grid* grid,
@@ -736,7 +744,7 @@ iso_status iso_extract_device(iso_ctx* ctx, iso_algorithm algo, const float* vol
     if (st != ISO_OK) return st;
     out->n_points = out->n_tris = 0;
     int64_t* res = reinterpret_cast<int64_t*>(ctx->h_totals);
-    st = iso_extract_device_async(ctx, algo, volume, grid, isoval, out, res, stream);
+    st = extract_device(ctx, algo, volume, grid, isoval, out, res, stream, true);
     if (st != ISO_OK) return st;
     ISO_CUDA(ctx, cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
     return finish_counts(ctx, out, res[0], res[1], res[3], &out->n_points, &out->n_tris);
@@ -862,9 +870,9 @@ static iso_status extract_device_narrow(iso_ctx* ctx, iso_algorithm algo, const 
     const long long capT = out->cap_tris;
     const bool i4 = out->index_bytes == 4;
     PassMarks pm(ctx, s);
-    iso::launch_count_narrow(volume, dtype, g, isoval, mc, pl.cp, b, s);
+    iso::launch_count_narrow(volume, dtype, g, isoval, mc, pl.cp, b, s, false);
     pm.mark(ISO_PASS_COUNT);
-    iso::launch_scan(g, pl.cp, mc ? iso::kScanMC : iso::kScanFE, b, s);
+    iso::launch_scan(g, pl.cp, mc ? iso::kScanMC : iso::kScanFE, b, s, ctx->h_totals);
     pm.mark(ISO_PASS_SCAN);
     if (!mc) {
         if (i4)
@@ -897,8 +905,7 @@ static iso_status extract_device_narrow(iso_ctx* ctx, iso_algorithm algo, const 
         pm.mark(ISO_PASS_MC_TRIANGLES);
     }
     ISO_CUDA(ctx, cudaGetLastError());
-    int64_t* res = reinterpret_cast<int64_t*>(ctx->h_totals);
-    ISO_CUDA(ctx, cudaMemcpyAsync(res, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    const int64_t* res = reinterpret_cast<const int64_t*>(ctx->h_totals);
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
     return finish_counts(ctx, out, res[0], res[1], res[3], &out->n_points, &out->n_tris);
 }

@@ -193,13 +193,13 @@ inline void carve(void* base, const Grid& g, const iso::CountPlan& cp, FeBuffers
 {
     const size_t R = (size_t)g.R;
     char* p = static_cast<char*>(base);
+    b.totals = reinterpret_cast<unsigned long long*>(p); p += align256(8 * 8);  // at one place whatever the grid
     b.rowcnt = reinterpret_cast<uint4*>(p); p += align256(R * 16);
     b.row4 = reinterpret_cast<uint4*>(p); p += align256(R * 16);
     b.trims = reinterpret_cast<uint2*>(p); p += align256(R * 8);
     b.mccnt = reinterpret_cast<uint32_t*>(p); p += align256(R * 4);
     b.starts = reinterpret_cast<unsigned long long*>(p); p += align256(4 * R * 8);
     b.part = reinterpret_cast<unsigned long long*>(p); p += align256(4 * (size_t)cp.nseg * 8);
-    b.totals = reinterpret_cast<unsigned long long*>(p); p += align256(8 * 8);
     b.bits = reinterpret_cast<uint32_t*>(p);
 }
 
@@ -216,6 +216,7 @@ inline iso_status ensure_scratch(iso_ctx* ctx, const Grid& g, const iso::CountPl
         const size_t alloc = need + need / 4;
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch, alloc));
         ctx->scratch_bytes = alloc;
+        ISO_CUDA(ctx, cudaMemsetAsync(ctx->scratch, 0, 8 * sizeof(unsigned long long), s));  // the device status
     }
     carve(ctx->scratch, g, cp, b);
     b.fe2mc = ctx->fe2mc;
@@ -250,6 +251,7 @@ inline iso_status ensure_scratch_b(iso_ctx* ctx, const Grid& g, const iso::Count
         const size_t alloc = need + need / 4;
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch_b, alloc));
         ctx->scratch_b_bytes = alloc;
+        ISO_CUDA(ctx, cudaMemsetAsync(ctx->scratch_b, 0, 8 * sizeof(unsigned long long), s));
     }
     carve(ctx->scratch_b, g, cp, b);
     b.fe2mc = ctx->fe2mc;
@@ -334,14 +336,15 @@ inline Plans make_plans(const iso_ctx* ctx, const Grid& g, int nsm = 0)
     return p;
 }
 
-// Passes 1-3: counts, scan, row starts.
+// Passes 1-3: counts, scan, row starts.  publish: the counts and the device status go there without a copy (pinned
+// host memory); the status is then the context's scratch's own, zero from call to call, and needs no memset.
 inline void enqueue_count(iso_ctx* ctx, iso_algorithm algo, const float* vol, const Grid& g, float iso, const Plans& pl,
-                   FeBuffers& b, cudaStream_t s, PassMarks& pm)
+                   FeBuffers& b, cudaStream_t s, PassMarks& pm, unsigned long long* publish = nullptr)
 {
     const bool mc = algo == ISO_MARCHING_CUBES;
-    iso::launch_count(vol, g, iso, ctx->d_cases, mc, pl.cp, b, s);
+    iso::launch_count(vol, g, iso, ctx->d_cases, mc, pl.cp, b, s, publish == nullptr);
     pm.mark(ISO_PASS_COUNT);
-    iso::launch_scan(g, pl.cp, algo == ISO_MC_DUPFREE ? iso::kScanDup : (mc ? iso::kScanMC : iso::kScanFE), b, s);
+    iso::launch_scan(g, pl.cp, algo == ISO_MC_DUPFREE ? iso::kScanDup : (mc ? iso::kScanMC : iso::kScanFE), b, s, publish);
     pm.mark(ISO_PASS_SCAN);
 }
 

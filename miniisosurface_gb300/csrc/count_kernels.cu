@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(kCountThreads) k_count_rows(const float* __res
 {
     extern __shared__ __align__(128) unsigned char s_raw[];
     __shared__ uint64_t s_bar[kCountWarps];
+    next_may_start();
     const int warp = threadIdx.x >> 5;
     const unsigned item = blockIdx.x * kCountWarps + warp;
     if (item >= nitems) return;
@@ -378,7 +379,25 @@ __global__ void __launch_bounds__(kThreads) k_scan_partial(const uint4* __restri
                                                            const uint32_t* __restrict__ mccnt, long long R,
                                                            unsigned long long* __restrict__ part, int nseg)
 {
+    wait_for_previous();
+    next_may_start();
     scan_partial_block<SM>(rowcnt, mccnt, R, part, nseg, (int)blockIdx.x);
+}
+
+// The totals' other duties, by one thread of the scan: the work counter of pass 4 starts at zero, and the counts go
+// to the host (launch_scan).
+__device__ __forceinline__ void scan_publish(unsigned long long* __restrict__ totals, unsigned long long v,
+                                             unsigned long long t, unsigned long long m,
+                                             unsigned long long* __restrict__ publish)
+{
+    totals[7] = 0;
+    if (publish) {
+        publish[0] = v;
+        publish[1] = t;
+        publish[2] = m;
+        publish[3] = totals[3];
+        totals[3] = 0;
+    }
 }
 
 // Segment blk: the starts of its rows from the segments' totals; segment 0 also writes the totals.
@@ -387,7 +406,8 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
                                                  const uint32_t* __restrict__ mccnt, long long R,
                                                  const unsigned long long* __restrict__ part, int nseg,
                                                  unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
-                                                 unsigned long long* __restrict__ totals, int blk)
+                                                 unsigned long long* __restrict__ totals,
+                                                 unsigned long long* __restrict__ publish, int blk)
 {
     constexpr int NC = ScanComps<SM>::n;
     __shared__ unsigned long long s_w[NC][kThreads / 32];
@@ -435,6 +455,8 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
         } else {
             for (int a = 0; a < 3; ++a) totals[a] = s_tot[a];
         }
+        scan_publish(totals, SM == kScanDup ? s_tot[0] + s_tot[2] + s_tot[3] : s_tot[0], s_tot[1],
+                     SM == kScanDup ? 0ull : s_tot[2], publish);
     }
 #pragma unroll
     for (int a = 0; a < NC; ++a) {
@@ -459,9 +481,100 @@ __global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* __restrict
                                                          const unsigned long long* __restrict__ part, int nseg,
                                                          unsigned long long* __restrict__ starts,
                                                          uint4* __restrict__ row4,
-                                                         unsigned long long* __restrict__ totals)
+                                                         unsigned long long* __restrict__ totals,
+                                                         unsigned long long* __restrict__ publish)
 {
-    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, row4, totals, (int)blockIdx.x);
+    wait_for_previous();
+    next_may_start();
+    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, row4, totals, publish, (int)blockIdx.x);
+}
+
+// The whole scan of a small grid in one CTA: one launch less than the two above where launches are most of the time.
+// A warp takes a run of 128 consecutive rows, a lane every 32nd of them, read once.  Events around the pass, us: 64^3
+// (4,096 rows) 9.0 against 11.4 with the two; at 16,384 rows (128^3) one CTA takes 18, the two 10.
+constexpr int kScanSmallPer = 4;
+constexpr long long kScanSmall = 1024ll * kScanSmallPer;
+
+template <int SM>
+__global__ void __launch_bounds__(1024) k_scan_small(const uint4* __restrict__ rowcnt,
+                                                     const uint32_t* __restrict__ mccnt, int R,
+                                                     unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
+                                                     unsigned long long* __restrict__ totals,
+                                                     unsigned long long* __restrict__ publish)
+{
+    constexpr int NC = SM == kScanFE ? 2 : ScanComps<SM>::n, PER = kScanSmallPer;
+    __shared__ uint32_t s_w[NC][32];
+    wait_for_previous();
+    next_may_start();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int r0 = warp * PER * 32 + lane;
+    uint32_t v[NC][PER], cx[PER], cxy[PER], sum[NC];  // 32 bits hold the counts of so many rows (scan_launch)
+#pragma unroll
+    for (int a = 0; a < NC; ++a) sum[a] = 0u;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int r = r0 + 32 * q;
+        const uint4 c = r < R ? __ldg(&rowcnt[r]) : make_uint4(0u, 0u, 0u, 0u);
+        cx[q] = c.x;
+        cxy[q] = c.x + c.y;
+        v[0][q] = SM == kScanDup ? c.x : c.x + c.y + c.z;
+        v[1][q] = c.w;
+        if (NC > 2) v[NC > 2 ? 2 : 0][q] = SM == kScanDup ? c.y : (r < R ? __ldg(&mccnt[r]) : 0u);
+        if (NC > 3) v[NC > 3 ? 3 : 0][q] = c.z;
+#pragma unroll
+        for (int a = 0; a < NC; ++a) sum[a] += v[a][q];
+    }
+#pragma unroll
+    for (int a = 0; a < NC; ++a) {
+        const uint32_t w = __reduce_add_sync(0xffffffffu, sum[a]);
+        if (lane == 0) s_w[a][warp] = w;
+    }
+    __syncthreads();
+    if (warp < NC) {  // warp a: the warps' sums before each; the last lane's end with the totals
+        const uint32_t x = s_w[warp][lane];
+        uint32_t inc = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += y;
+        }
+        s_w[warp][lane] = inc - x;
+    }
+    __syncthreads();
+    uint32_t run[NC];
+#pragma unroll
+    for (int a = 0; a < NC; ++a) run[a] = s_w[a][warp];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const int r = r0 + 32 * q;
+#pragma unroll
+        for (int a = 0; a < NC; ++a) {
+            uint32_t inc = v[a][q];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += y;
+            }
+            const uint32_t first = run[a] + inc - v[a][q];
+            if (r < R) {
+                starts[(long long)a * R + r] = first;
+                if (SM != kScanDup && a == 0) row4[r] = make_uint4(first, first + cx[q], first + cxy[q], 0u);
+            }
+            run[a] += __shfl_sync(0xffffffffu, inc, 31);
+        }
+    }
+    if (t == 1023) {
+        const unsigned long long e2 = NC > 2 ? run[NC > 2 ? 2 : 0] : 0u, e3 = NC > 3 ? run[NC > 3 ? 3 : 0] : 0u;
+        const unsigned long long V = SM == kScanDup ? run[0] + e2 + e3 : run[0], m = SM == kScanDup ? 0ull : e2;
+        totals[0] = V;
+        totals[1] = run[1];
+        totals[2] = m;
+        if (SM == kScanDup) {
+            totals[4] = run[0];
+            totals[5] = e2;
+        }
+        scan_publish(totals, V, run[1], m, publish);
+    }
 }
 
 // The Flying Edges scans of a list of requests, one launch per phase: block x is segment
@@ -486,7 +599,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_final_batch(const BatchReq* _
     const int blk = (int)(blockIdx.x - __ldg(&first[q]));
     if (blk >= d->nseg) return;
     scan_final_block<kScanFE>(d->rowcnt, nullptr, d->g.R, d->part, d->nseg, d->starts, d->row4,
-                              d->totals, blk);
+                              d->totals, nullptr, blk);
 }
 
 // vfirst[q] = the vertices of requests list[0 .. q-1] whose meshes hold their counts (one CTA of 1024 threads,
@@ -713,9 +826,9 @@ static void count_launch(const CountPlan& p, const float* vol, const Grid& g, fl
 }
 
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
-                  const CountPlan& p, FeBuffers& b, cudaStream_t s)
+                  const CountPlan& p, FeBuffers& b, cudaStream_t s, bool zero_status)
 {
-    cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
+    if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
     if (mc) count_launch<true>(p, vol, g, iso, cases, b, s);
     else count_launch<false>(p, vol, g, iso, cases, b, s);
 }
@@ -759,19 +872,24 @@ void launch_place_batch(BatchReq* reqs, const int* list, int m, const PackedOut&
     k_batch_place<<<1, 1024, 0, s>>>(reqs, list, m, out, vfirst);
 }
 
-void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s)
+template <int SM>
+static void scan_launch(const Grid& g, const CountPlan& p, FeBuffers& b, cudaStream_t s, unsigned long long* publish)
 {
-#define ISO_SCAN(SM)                                                                                            \
-    k_scan_partial<SM><<<p.nseg, kThreads, 0, s>>>(b.rowcnt, b.mccnt, g.R, b.part, p.nseg);                      \
-    k_scan_final<SM><<<p.nseg, kThreads, 0, s>>>(b.rowcnt, b.mccnt, g.R, b.part, p.nseg, b.starts, b.row4, b.totals)
-    if (mode == kScanMC) {
-        ISO_SCAN(kScanMC);
-    } else if (mode == kScanDup) {
-        ISO_SCAN(kScanDup);
-    } else {
-        ISO_SCAN(kScanFE);
+    if (g.R <= kScanSmall && g.nx <= (1 << 15)) {  // their triangles stay below 2^32
+        launch_after(k_scan_small<SM>, 1, 1024, 0, s, b.rowcnt, b.mccnt, (int)g.R, b.starts, b.row4, b.totals, publish);
+        return;
     }
-#undef ISO_SCAN
+    launch_after(k_scan_partial<SM>, p.nseg, kThreads, 0, s, b.rowcnt, b.mccnt, g.R, b.part, p.nseg);
+    launch_after(k_scan_final<SM>, p.nseg, kThreads, 0, s, b.rowcnt, b.mccnt, g.R, b.part, p.nseg, b.starts, b.row4,
+                 b.totals, publish);
+}
+
+void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,
+                 unsigned long long* publish)
+{
+    if (mode == kScanMC) scan_launch<kScanMC>(g, p, b, s, publish);
+    else if (mode == kScanDup) scan_launch<kScanDup>(g, p, b, s, publish);
+    else scan_launch<kScanFE>(g, p, b, s, publish);
 }
 
 RowStarts row_starts(const Grid& g, const CountPlan& p, const FeBuffers& b)

@@ -219,9 +219,9 @@ static void narrow_launch(const CountPlan& p, const S* vol, const Grid& g, int t
 }
 
 void launch_count_narrow(const void* vol, int dtype, const Grid& g, float iso, bool mc, const CountPlan& p, FeBuffers& b,
-                         cudaStream_t s)
+                         cudaStream_t s, bool zero_status)
 {
-    cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
+    if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
     const int thr = narrow_threshold(iso);
 #define ISO_TYPE(T)                                                                   \
     {                                                                                 \

@@ -431,6 +431,8 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells(
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ GenCellTables<MODE> tabs;
     stage_gen_tables<MODE>(cases, tabs);
+    wait_for_previous();
+    next_may_start();
     __syncthreads();  // the only CTA barrier: from here on every warp runs alone
     // Caller grows buffers.  Past this check every record slot and triangle index written below lies
     // under the totals, because the count pass derives the counts and starts from the same bit words
@@ -482,11 +484,12 @@ inline int gen_cells_warps(int ws_bytes, size_t fixed)
     return (int)std::max(1ll, std::min<long long>(kGenMaxWarps, room / ws_bytes));
 }
 
-// Rows of up to 32 words (gen_plan's fits) in MODE over the plan's planes [kbeg, kend).
+// Rows of up to 32 words (gen_plan's fits) in MODE over the plan's planes [kbeg, kend).  again: not the first such
+// launch since the scan, which leaves the work counter at zero.
 template <typename IndexT, int MODE>
 void launch_gen_cells(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                       const GenPlan& p, long long capV, long long capT, float* points, IndexT* tris, int reverse,
-                      cudaStream_t s)
+                      cudaStream_t s, bool again = false)
 {
     const int nzw = p.kend - p.kbeg;
     if (nzw <= 0) return;
@@ -517,13 +520,13 @@ void launch_gen_cells(const Grid& g, const CaseTables* cases, const FeBuffers& b
     RowStarts rs = row_starts(g, cp, b);
     for (int a = 0; a < 3; ++a) rs.add[a] = p.add[a];
     unsigned int* work = reinterpret_cast<unsigned int*>(b.totals + 7);
-    cudaMemsetAsync(work, 0, sizeof(unsigned int), s);
+    if (again) cudaMemsetAsync(work, 0, sizeof(unsigned int), s);
     const size_t smem = (size_t)warps * ws_bytes;
     auto kern = rpw == 1 ? k_gen_cells<IndexT, MODE, 1> : (rpw == 2 ? k_gen_cells<IndexT, MODE, 2> : k_gen_cells<IndexT, MODE, 0>);
     allow_smem(kern, smem);
-    kern<<<(unsigned)blocks, 32 * warps, smem, s>>>(b.bits, g, rpw, cols, (int)ngroups, (uint32_t)nitems, p.kbeg, p.kend, p.kemit,
-                                                    p.vbase, p.tbase, ws_bytes, cases, b.row4, rs, b.totals, work,
-                                                    capV, capT, points, tris, b.fe2mc, reverse);
+    launch_after(kern, (unsigned)blocks, 32u * warps, smem, s, b.bits, g, rpw, cols, (int)ngroups, (uint32_t)nitems,
+                 p.kbeg, p.kend, p.kemit, p.vbase, p.tbase, ws_bytes, cases, b.row4, rs, b.totals, work, capV, capT,
+                 points, tris, b.fe2mc, reverse);
 }
 
 }  // namespace iso

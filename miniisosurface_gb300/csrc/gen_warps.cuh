@@ -410,7 +410,6 @@ void launch_gen_dup(const Grid& g, const CaseTables* cases, const FeBuffers& b, 
     const long long nitems = (long long)g.ny * nkc;
     const long long blocks = std::min((nitems + kGenRows - 1) / kGenRows, (long long)p.nsm * kGenCtasPerSm);
     unsigned int* work = reinterpret_cast<unsigned int*>(b.totals + 7);
-    cudaMemsetAsync(work, 0, sizeof(unsigned int), s);
     const int ws_bytes = (int)gen_warp_scratch_bytes(g.W);
     const size_t smem = (size_t)kGenRows * ws_bytes;
     auto kern = k_gen_warps<IndexT>;

@@ -107,6 +107,7 @@ template <typename IndexT, bool VEC>
 __global__ void k_mc_remap(IndexT* __restrict__ tris, const uint32_t* __restrict__ fe2mc,
                            const unsigned long long* __restrict__ totals, long long capV, long long capT)
 {
+    wait_for_previous();
     if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
     const unsigned long long n = 3ull * totals[1];
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -144,9 +145,9 @@ void launch_mc_remap(const FeBuffers& b, const GenPlan& p, long long capV, long 
     const long long need = (3 * capT / (4 * kRemapUnroll) + kThreads - 1) / kThreads;
     const unsigned blocks = (unsigned)std::max(1ll, std::min(wave, need));
     if ((reinterpret_cast<uintptr_t>(tris) & 15) == 0)
-        k_mc_remap<IndexT, true><<<blocks, kThreads, 0, s>>>(tris, b.fe2mc, b.totals, capV, capT);
+        launch_after(k_mc_remap<IndexT, true>, blocks, kThreads, 0, s, tris, b.fe2mc, b.totals, capV, capT);
     else
-        k_mc_remap<IndexT, false><<<blocks, kThreads, 0, s>>>(tris, b.fe2mc, b.totals, capV, capT);
+        launch_after(k_mc_remap<IndexT, false>, blocks, kThreads, 0, s, tris, b.fe2mc, b.totals, capV, capT);
 }
 
 template void launch_mc_gen_tris<uint32_t>(const Grid&, const CaseTables*, const FeBuffers&, const CountPlan&,
@@ -164,7 +165,7 @@ template <typename IndexT>
 void launch_mc_tri_warps(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                          const GenPlan& p, long long capV, long long capT, IndexT* tris, cudaStream_t s)
 {
-    launch_gen_cells<IndexT, kGenTri>(g, cases, b, cp, p, capV, capT, nullptr, tris, 0, s);
+    launch_gen_cells<IndexT, kGenTri>(g, cases, b, cp, p, capV, capT, nullptr, tris, 0, s, true);
 }
 
 template <typename IndexT>

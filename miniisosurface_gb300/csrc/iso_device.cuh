@@ -515,6 +515,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
 #endif
 }
 
+// A kernel launched beside its predecessor in the stream (launch_after) waits
+// here for that one's end before it reads or writes anything of it; every thread
+// of every such kernel comes by, so that a kernel's end implies its
+// predecessors'.  next_may_start lets the successor be brought in meanwhile.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // First vertex (comp 0), triangle (1) or MC vertex (2) of grid row r =
 // k*ny + j, from the scanned starts[3][R].
 // Window row r (see Grid); add[comp] shifts the window's numbering to the

@@ -2,6 +2,7 @@
 #pragma once
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -78,15 +79,38 @@ inline void allow_smem(K kern, size_t dyn)
     if (dyn > cur && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) == cudaSuccess)
         cur = dyn;
 }
+
+// Launches kern so that it may be brought onto the device while the kernel before it in the stream ends (its first
+// statement then is wait_for_previous, iso_device.cuh): the launch and the staging of tables overlap that end.
+template <typename... P, typename... A>
+inline void launch_after(void (*kern)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t s, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, P(std::forward<A>(args))...);
+}
+
 CountPlan count_plan(const Grid& g, int nsm);
 CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned, bool trims);
 GenPlan gen_plan(const Grid& g, int nsm);
 
 // passes 1-3
+// zero_status: the device status (totals[3]) is zeroed first; without it, it has to be zero (launch_scan's publish)
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
-                  const CountPlan& p, FeBuffers& b, cudaStream_t s);
+                  const CountPlan& p, FeBuffers& b, cudaStream_t s, bool zero_status = true);
 enum ScanMode { kScanFE = 0, kScanMC = 1, kScanDup = 2 };
-void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s);
+// Row starts and totals; the work counter of pass 4 (totals[7]) zeroed.  publish (device-visible host memory, or null):
+// the totals and the device status are also written there, and the status is zero again for the next count.
+void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,
+                 unsigned long long* publish = nullptr);
 // totals and the starts of rows rlo / rhi into out[0..8] (device-visible host memory)
 void launch_slab_readback(const FeBuffers& b, const Grid& g, long long rlo, long long rhi, bool has_lo, bool has_hi,
                           unsigned long long* out, cudaStream_t s);
@@ -122,7 +146,7 @@ void launch_fe_gen_warps(const float* vol, const Grid& g, float iso, const CaseT
 // generate pass, then the vertex pass over the same samples.
 bool narrow_fits(const Grid& g, const void* vol, int dtype);
 void launch_count_narrow(const void* vol, int dtype, const Grid& g, float iso, bool mc, const CountPlan& p,
-                         FeBuffers& b, cudaStream_t s);
+                         FeBuffers& b, cudaStream_t s, bool zero_status = true);
 bool launch_fe_vertices_narrow(const void* vol, int dtype, const Grid& g, float iso, const FeBuffers& b,
                                const GenPlan& p, long long capV, long long capT, float* points, float* normals,
                                cudaStream_t s);
