@@ -163,105 +163,147 @@ __global__ void k_block_tris(const uint32_t* __restrict__ bits, Grid g, BlockDim
 }
 
 // ---- the network -----------------------------------------------------------
-// A CTA of 256 threads takes tiles of 64 samples.  Thread t works on sample
-// row r = t / 4 and the 16 hidden units u0 .. u0 + 15, u0 = 16 * (t % 4), for
-// the layer products; the weight gradients accumulate in registers over all
-// tiles of the CTA (dW2 row i = t / 4, dW1 row k = t / 4 for t < 4 * kIn)
-// and are added to `grads` once at the end.  Shared rows are padded to 65
-// floats so that columns spread over the banks.
-constexpr int kTile = 64, kPad = kHid + 1, kXPad = kIn + 1;
+// A CTA of 512 threads takes tiles of 64 samples.  Everything that is summed over
+// is the slow index in shared memory (x, h1, d2, d1 by input or unit, 64 samples
+// side by side; the weights by input, 64 units side by side), so that a thread
+// makes a 4 x 2 part of a product from a 16-byte and an 8-byte load per term: warp
+// w the samples 4 w on, lane l the units 2 l and 2 l + 1.  The weight gradients are
+// sums over the samples: a thread makes those of units w + 16 a by l + 32 b from
+// 16-byte loads of four samples, in registers over all tiles of the CTA; eight
+// CTAs of a cluster then add theirs up through distributed shared memory, so that
+// a gradient gets one global addition per cluster instead of one per CTA (1.6
+// million on 6,401 addresses for 16,384 samples).  Sums are fused multiply-adds.
+// What bounds it, for 16,384 samples (256 tiles; 38 us, 106 with a row of 16 units
+// per thread and every CTA's own additions): issue in the tiles (24 us, 57 thousand
+// instructions each), latency in the rest (the weights' way in, five barriers a
+// tile, the cluster's end: 13 us).  Half the threads with 4 x 4 parts: 41 us.
+constexpr int kTile = 64, kRow = kTile + 4;  // samples of a tile; of a row in shared memory (16-byte aligned)
+constexpr int kMlpCluster = 8;
+constexpr int kUnitRow = kHid + 2;
+constexpr int kMlpThreads = 512;
 
-struct MlpSmem {
-    float w1[kIn * kHid], b1[kHid], w2[kHid * kPad], b2[kHid], w3[kHid], b3;
-    float x[kTile * kXPad], h1[kTile * kPad], h2[kTile * kPad], d2[kTile * kPad], d1[kTile * kPad];
-    float dy[kTile], y[kTile];
+struct __align__(16) MlpSmem {
+    float w1[kIn * kHid], w2[kHid * kHid], b1[kHid], b2[kHid], w3[kHid], b3[4];
+    float x[kIn * kRow], h1[kHid * kRow];
+    float y[kTile];
 };
+
+struct __align__(16) MlpGradSmem {
+    MlpSmem f;
+    float w2t[kHid * kUnitRow];             // w2 by unit of the second layer, rows two floats apart in the banks
+    float d2[kHid * kRow], d1[kHid * kRow];
+    float dy[kTile], w3p[16 * kHid];        // each warp's part of dW3
+};
+static_assert(sizeof(float) * kParams <= sizeof(float) * 2 * kHid * kRow, "a CTA's gradients fit over d2 and d1");
 
 __device__ __forceinline__ void load_params(MlpSmem& s, const float* __restrict__ p)
 {
     for (int i = threadIdx.x; i < kIn * kHid; i += blockDim.x) s.w1[i] = p[i];
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.w2[(i / kHid) * kPad + i % kHid] = p[kOffW2 + i];
+    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.w2[i] = p[kOffW2 + i];
     for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
         s.b1[i] = p[kOffB1 + i];
         s.b2[i] = p[kOffB2 + i];
         s.w3[i] = p[kOffW3 + i];
     }
-    if (threadIdx.x == 0) s.b3 = p[kOffB3];
+    if (threadIdx.x == 0) s.b3[0] = p[kOffB3];
 }
 
-// Inputs of sample n for the isovalue iso[n] from its block statistics.
+// Input c of a block's statistics st for the isovalue iso.
+__device__ __forceinline__ float mlp_input(const float* __restrict__ st, float iso, int c)
+{
+    if (c >= 2) return st[c];
+    const float range = st[1] - st[0];
+    return range > 0.f ? (st[c] - iso) / range : 0.f;
+}
+
+// Inputs of the tile's samples from their block statistics.
 __device__ __forceinline__ void load_tile(MlpSmem& s, const float* __restrict__ stats, const float* __restrict__ iso,
                                           long long base, long long n)
 {
     for (int i = threadIdx.x; i < kTile * kIn; i += blockDim.x) {
         const int r = i / kIn, c = i % kIn;
         const long long q = base + r;
-        float v = 0.f;
-        if (q < n) {
-            const float* st = stats + q * kIn;
-            if (c < 2) {
-                const float range = st[1] - st[0];
-                v = range > 0.f ? (st[c] - iso[q]) / range : 0.f;
-            } else {
-                v = st[c];
-            }
-        }
-        s.x[r * kXPad + c] = v;
+        s.x[c * kRow + r] = q < n ? mlp_input(stats + q * kIn, iso[q], c) : 0.f;
     }
 }
 
-// h1, h2 and the output y of the tile.
-__device__ __forceinline__ void forward_tile(MlpSmem& s)
+// out[b][a] = the product's value for sample r0 + a and unit c0 + b: bias + sum over K of in[k][sample] w[k][unit].
+template <int K, int WROW = kHid>
+__device__ __forceinline__ void mlp_product(const float* in, const float* w, const float* bias, int r0, int c0,
+                                            float (&out)[2][4])
 {
-    const int r = threadIdx.x >> 2, u0 = 16 * (threadIdx.x & 3);
-    float acc[16];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) acc[q] = s.b1[u0 + q];
-    for (int k = 0; k < kIn; ++k) {
-        const float xv = s.x[r * kXPad + k];
+    for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] += xv * s.w1[k * kHid + u0 + q];
+        for (int a = 0; a < 4; ++a) out[b][a] = bias ? bias[c0 + b] : 0.f;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+        const float4 xv = *reinterpret_cast<const float4*>(in + k * kRow + r0);
+        const float2 wv = *reinterpret_cast<const float2*>(w + k * WROW + c0);
+        const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[2] = {wv.x, wv.y};
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int a = 0; a < 4; ++a) out[b][a] = __fmaf_rn(xs[a], ws[b], out[b][a]);
     }
+}
+
+__device__ __forceinline__ void store_units(float* o, int r0, int c0, const float (&v)[2][4])
+{
 #pragma unroll
-    for (int q = 0; q < 16; ++q) s.h1[r * kPad + u0 + q] = fmaxf(acc[q], 0.f);
+    for (int b = 0; b < 2; ++b)
+        *reinterpret_cast<float4*>(o + (c0 + b) * kRow + r0) = make_float4(v[b][0], v[b][1], v[b][2], v[b][3]);
+}
+
+// h1 (in shared memory), h2 (the thread's 4 x 2 part) and the output y of the tile.
+__device__ __forceinline__ void forward_tile(MlpSmem& s, float (&h2)[2][4])
+{
+    const int r0 = 4 * (threadIdx.x >> 5), c0 = 2 * (threadIdx.x & 31);
+    float h1[2][4];
+    mlp_product<kIn>(s.x, s.w1, s.b1, r0, c0, h1);
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) h1[b][a] = fmaxf(h1[b][a], 0.f);
+    store_units(s.h1, r0, c0, h1);
     __syncthreads();
+    mlp_product<kHid>(s.h1, s.w2, s.b2, r0, c0, h2);
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int q = 0; q < 16; ++q) acc[q] = s.b2[u0 + q];
-    for (int i = 0; i < kHid; ++i) {
-        const float hv = s.h1[r * kPad + i];
+    for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] += hv * s.w2[i * kPad + u0 + q];
-    }
+        for (int a = 0; a < 4; ++a) {
+            h2[b][a] = fmaxf(h2[b][a], 0.f);
+            part[a] = __fmaf_rn(h2[b][a], s.w3[c0 + b], part[a]);
+        }
 #pragma unroll
-    for (int q = 0; q < 16; ++q) s.h2[r * kPad + u0 + q] = fmaxf(acc[q], 0.f);
-    __syncthreads();
-    if (threadIdx.x < kTile) {
-        float y = s.b3;
-        for (int u = 0; u < kHid; ++u) y += s.h2[threadIdx.x * kPad + u] * s.w3[u];
-        s.y[threadIdx.x] = y;
+    for (int a = 0; a < 4; ++a) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) part[a] += __shfl_xor_sync(0xffffffffu, part[a], d);
+        if ((threadIdx.x & 31) == 0) s.y[r0 + a] = part[a] + s.b3[0];
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_mlp_forward(const float* __restrict__ params, const float* __restrict__ stats,
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(const float* __restrict__ params, const float* __restrict__ stats,
                                                      const float* __restrict__ iso, long long n, float* __restrict__ y)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     MlpSmem& s = *reinterpret_cast<MlpSmem*>(s_raw);
     load_params(s, params);
-    __syncthreads();
     for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
         load_tile(s, stats, iso, base, n);
         __syncthreads();
-        forward_tile(s);
+        float h2[2][4];
+        forward_tile(s, h2);
         if (threadIdx.x < kTile && base + threadIdx.x < n) y[base + threadIdx.x] = s.y[threadIdx.x];
-        __syncthreads();
     }
 }
 
 // Prediction for many (block statistics, isovalue) sets in one launch: the
 // samples are the sets' blocks one after another; a block counts when
-// min < iso <= max, and max(y, 0) of those is added to its set's total.
+// min < iso <= max, and max(y, 0) of those is added to its set's total.  A tile's
+// samples of one set are summed before the global addition.
 constexpr int kMaxSets = 128;
 struct PredictSets {
     int n;
@@ -270,14 +312,13 @@ struct PredictSets {
     float iso[kMaxSets];
 };
 
-__global__ void __launch_bounds__(256) k_mlp_predict(const float* __restrict__ params, PredictSets sets,
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_predict(const float* __restrict__ params, PredictSets sets,
                                                      float* __restrict__ totals)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     MlpSmem& s = *reinterpret_cast<MlpSmem*>(s_raw);
     __shared__ int s_set[kTile];
     load_params(s, params);
-    __syncthreads();
     const long long n = sets.start[sets.n];
     for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
         if (threadIdx.x < kTile) {  // the set of sample base + t (-1: past the end or an inactive block)
@@ -295,26 +336,29 @@ __global__ void __launch_bounds__(256) k_mlp_predict(const float* __restrict__ p
             }
             s_set[threadIdx.x] = set;
         }
-        __syncthreads();
+        if (!__syncthreads_or(threadIdx.x < kTile && s_set[threadIdx.x] >= 0)) continue;  // no active block
         for (int i = threadIdx.x; i < kTile * kIn; i += blockDim.x) {
             const int r = i / kIn, c = i % kIn;
             const int set = s_set[r];
-            float v = 0.f;
-            if (set >= 0) {
-                const float* st = sets.stats[set] + (base + r - sets.start[set]) * kIn;
-                if (c < 2) {
-                    const float range = st[1] - st[0];
-                    v = range > 0.f ? (st[c] - sets.iso[set]) / range : 0.f;
-                } else {
-                    v = st[c];
-                }
-            }
-            s.x[r * kXPad + c] = v;
+            s.x[c * kRow + r] =
+                set >= 0 ? mlp_input(sets.stats[set] + (base + r - sets.start[set]) * kIn, sets.iso[set], c) : 0.f;
         }
         __syncthreads();
-        forward_tile(s);
-        if (threadIdx.x < kTile && s_set[threadIdx.x] >= 0)
-            atomicAdd(&totals[s_set[threadIdx.x]], fmaxf(s.y[threadIdx.x], 0.f));
+        float h2[2][4];
+        forward_tile(s, h2);
+        if (threadIdx.x < 32) {  // the sets of a tile are neighbours
+            const int lane = threadIdx.x, a = s_set[lane], b = s_set[lane + 32];
+            const float ya = a >= 0 ? fmaxf(s.y[lane], 0.f) : 0.f, yb = b >= 0 ? fmaxf(s.y[lane + 32], 0.f) : 0.f;
+            const int none = sets.n;
+            int q = __reduce_min_sync(0xffffffffu, min(a >= 0 ? a : none, b >= 0 ? b : none));
+            while (q < none) {
+                float v = (a == q ? ya : 0.f) + (b == q ? yb : 0.f);
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+                if (lane == 0) atomicAdd(&totals[q], v);
+                q = __reduce_min_sync(0xffffffffu, min(a > q ? a : none, b > q ? b : none));
+            }
+        }
         __syncthreads();
     }
 }
@@ -322,94 +366,158 @@ __global__ void __launch_bounds__(256) k_mlp_predict(const float* __restrict__ p
 // Gradient of the mean squared error (1/n) sum (y - target)^2 with respect
 // to every parameter, added into grads (zeroed by the caller); the loss
 // into *loss.
-__global__ void __launch_bounds__(256) k_mlp_gradient(const float* __restrict__ params,
-                                                      const float* __restrict__ stats, const float* __restrict__ iso,
-                                                      const float* __restrict__ target, long long n,
-                                                      float* __restrict__ grads, float* __restrict__ loss)
+__global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThreads, 2)
+    k_mlp_gradient(const float* __restrict__ params, const float* __restrict__ stats, const float* __restrict__ iso,
+                   const float* __restrict__ target, long long n, float* __restrict__ grads, float* __restrict__ loss)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    MlpSmem& s = *reinterpret_cast<MlpSmem*>(s_raw);
-    load_params(s, params);
-    __syncthreads();
-    const int t = threadIdx.x, r = t >> 2, u0 = 16 * (t & 3);
-    float gw2[16], gw1[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) gw2[q] = gw1[q] = 0.f;
-    float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, lsum = 0.f;
+    MlpGradSmem& s = *reinterpret_cast<MlpGradSmem*>(s_raw);
+    const int t = threadIdx.x, ty = t >> 5, tx = t & 31, r0 = 4 * ty, c0 = 2 * tx;
+    load_params(s.f, params);
+    for (int i = t; i < kHid * kHid; i += kMlpThreads) s.w2t[(i % kHid) * kUnitRow + i / kHid] = params[kOffW2 + i];
+    float gw2[4][2] = {}, gw1[3][2] = {}, gw3[2] = {};
+    float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, lsum = 0.f;
     const float inv_n = 1.f / (float)n;
     for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
-        load_tile(s, stats, iso, base, n);
+        load_tile(s.f, stats, iso, base, n);
         __syncthreads();
-        forward_tile(s);
+        float h2[2][4];
+        forward_tile(s.f, h2);
         if (t < kTile) {
             const long long q = base + t;
             float dy = 0.f;
             if (q < n) {
-                const float e = s.y[t] - target[q];
-                lsum += e * e;
+                const float e = s.f.y[t] - target[q];
+                lsum = __fmaf_rn(e, e, lsum);
                 dy = 2.f * e * inv_n;
             }
             s.dy[t] = dy;
+            gb3 += dy;
         }
         __syncthreads();
-        // d2 = dy * w3 where h2 > 0
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int u = u0 + q;
-            s.d2[r * kPad + u] = s.h2[r * kPad + u] > 0.f ? s.dy[r] * s.w3[u] : 0.f;
-        }
-        __syncthreads();
-        // d1[r][i] = sum_u d2[r][u] w2[i][u] where h1 > 0
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int i = u0 + q;
-            float acc = 0.f;
-            for (int u = 0; u < kHid; ++u) acc += s.d2[r * kPad + u] * s.w2[i * kPad + u];
-            s.d1[r * kPad + i] = s.h1[r * kPad + i] > 0.f ? acc : 0.f;
-        }
-        __syncthreads();
-        // weight gradients of the tile
+        // d2 = dy * w3 where h2 > 0; dW3 += h2 dy
+        float d[2][4];
         {
-            const int i = r;  // dW2 row
-            for (int rr = 0; rr < kTile; ++rr) {
-                const float hv = s.h1[rr * kPad + i];
+            const float4 dv = *reinterpret_cast<const float4*>(s.dy + r0);
+            const float dys[4] = {dv.x, dv.y, dv.z, dv.w};
 #pragma unroll
-                for (int q = 0; q < 16; ++q) gw2[q] += hv * s.d2[rr * kPad + u0 + q];
-            }
-        }
-        if (r < kIn) {
-            const int k = r;  // dW1 row
-            for (int rr = 0; rr < kTile; ++rr) {
-                const float xv = s.x[rr * kXPad + k];
+            for (int b = 0; b < 2; ++b)
 #pragma unroll
-                for (int q = 0; q < 16; ++q) gw1[q] += xv * s.d1[rr * kPad + u0 + q];
-            }
+                for (int a = 0; a < 4; ++a) {
+                    d[b][a] = h2[b][a] > 0.f ? dys[a] * s.f.w3[c0 + b] : 0.f;
+                    gw3[b] = __fmaf_rn(h2[b][a], dys[a], gw3[b]);
+                }
         }
-        if (t < kHid) {
-            for (int rr = 0; rr < kTile; ++rr) {
-                gb1 += s.d1[rr * kPad + t];
-                gb2 += s.d2[rr * kPad + t];
-                gw3 += s.h2[rr * kPad + t] * s.dy[rr];
-            }
-        }
-        if (t == 0)
-            for (int rr = 0; rr < kTile; ++rr) gb3 += s.dy[rr];
+        store_units(s.d2, r0, c0, d);
         __syncthreads();
-    }
+        // d1[sample][i] = sum_u d2[sample][u] w2[i][u] where h1 > 0
+        mlp_product<kHid, kUnitRow>(s.d2, s.w2t, nullptr, r0, c0, d);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) atomicAdd(&grads[kOffW2 + r * kHid + u0 + q], gw2[q]);
-    if (r < kIn) {
+        for (int b = 0; b < 2; ++b) {
+            const float4 hv = *reinterpret_cast<const float4*>(s.f.h1 + (c0 + b) * kRow + r0);
+            d[b][0] = hv.x > 0.f ? d[b][0] : 0.f;
+            d[b][1] = hv.y > 0.f ? d[b][1] : 0.f;
+            d[b][2] = hv.z > 0.f ? d[b][2] : 0.f;
+            d[b][3] = hv.w > 0.f ? d[b][3] : 0.f;
+        }
+        store_units(s.d1, r0, c0, d);
+        __syncthreads();
+        // the tile's weight gradients, four samples at a time
+#pragma unroll 2
+        for (int r = 0; r < kTile; r += 4) {
+            float4 hv[4], dv[2];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) atomicAdd(&grads[r * kHid + u0 + q], gw1[q]);
+            for (int a = 0; a < 4; ++a) hv[a] = *reinterpret_cast<const float4*>(s.f.h1 + (ty + 16 * a) * kRow + r);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dv[b] = *reinterpret_cast<const float4*>(s.d2 + (tx + 32 * b) * kRow + r);
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+                    gw2[a][b] = __fmaf_rn(hv[a].x, dv[b].x, __fmaf_rn(hv[a].y, dv[b].y, __fmaf_rn(hv[a].z, dv[b].z,
+                                          __fmaf_rn(hv[a].w, dv[b].w, gw2[a][b]))));
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                hv[a] = ty + 16 * a < kIn ? *reinterpret_cast<const float4*>(s.f.x + (ty + 16 * a) * kRow + r)
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dv[b] = *reinterpret_cast<const float4*>(s.d1 + (tx + 32 * b) * kRow + r);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+                    gw1[a][b] = __fmaf_rn(hv[a].x, dv[b].x, __fmaf_rn(hv[a].y, dv[b].y, __fmaf_rn(hv[a].z, dv[b].z,
+                                          __fmaf_rn(hv[a].w, dv[b].w, gw1[a][b]))));
+        }
+        if (t < 2 * kHid) {  // db1, db2: one unit's samples per thread
+            const float* row = t < kHid ? s.d1 + t * kRow : s.d2 + (t - kHid) * kRow;
+            float sum = 0.f;
+            for (int r = 0; r < kTile; r += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(row + r);
+                sum += (v.x + v.y) + (v.z + v.w);
+            }
+            if (t < kHid) gb1 += sum;
+            else gb2 += sum;
+        }
+        __syncthreads();  // the next tile overwrites x, h1, d2, d1
     }
+    // the CTA's gradients, in the parameters' layout, over d2 and d1
+    float* own = s.d2;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) own[kOffW2 + (ty + 16 * a) * kHid + tx + 32 * b] = gw2[a][b];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+            if (ty + 16 * a < kIn) own[(ty + 16 * a) * kHid + tx + 32 * b] = gw1[a][b];
+    if (t < kHid) own[kOffB1 + t] = gb1;
+    else if (t < 2 * kHid) own[kOffB2 + t - kHid] = gb2;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) s.w3p[ty * kHid + c0 + b] = gw3[b];  // dW3: the warps' parts
+    if (t < kTile) {  // db3 and the loss: two warps
+        for (int d = 16; d > 0; d >>= 1) {
+            gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
+            lsum += __shfl_xor_sync(0xffffffffu, lsum, d);
+        }
+        if ((t & 31) == 0) {
+            s.dy[t >> 5] = gb3;
+            s.dy[2 + (t >> 5)] = lsum;
+        }
+    }
+    __syncthreads();
     if (t < kHid) {
-        atomicAdd(&grads[kOffB1 + t], gb1);
-        atomicAdd(&grads[kOffB2 + t], gb2);
-        atomicAdd(&grads[kOffW3 + t], gw3);
+        float v = 0.f;
+        for (int w = 0; w < 16; ++w) v += s.w3p[w * kHid + t];
+        own[kOffW3 + t] = v;
     }
-    if (t == 0) atomicAdd(&grads[kOffB3], gb3);
-    for (int d = 16; d > 0; d >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, d);
-    if ((t & 31) == 0) atomicAdd(loss, lsum * inv_n);
+    if (t == kHid) {
+        own[kOffB3] = s.dy[0] + s.dy[1];
+        atomicAdd(loss, (s.dy[2] + s.dy[3]) * inv_n);
+    }
+    // every CTA of the cluster adds up its eighth of the parameters
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    constexpr int kShare = (kParams + kMlpCluster - 1) / kMlpCluster;
+    for (int i = t; i < kShare; i += kMlpThreads) {
+        const int q = (int)rank * kShare + i;
+        if (q < kParams) {
+            float sum = 0.f;
+#pragma unroll
+            for (uint32_t c = 0; c < kMlpCluster; ++c) {
+                uint32_t at;
+                float v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(own + q)), "r"(c));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+                sum += v;
+            }
+            if (sum != 0.f) atomicAdd(&grads[q], sum);
+        }
+    }
+    // no CTA ends while another reads its shared memory
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // Adam (Kingma & Ba 2015) with bias correction; step counts from 1.
@@ -429,10 +537,10 @@ __global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* 
 
 size_t mlp_smem() { return sizeof(MlpSmem); }
 
-int mlp_blocks(long long n, int nsm)
+int mlp_blocks(long long n, int nsm, int per_sm)
 {
     const long long tiles = (n + kTile - 1) / kTile;
-    return (int)std::min<long long>(tiles, (long long)nsm * 2);
+    return (int)std::min<long long>(tiles, (long long)nsm * per_sm);
 }
 
 int device_sms()
@@ -509,7 +617,7 @@ iso_status iso_mlp_forward(const float* params, const float* stats, const float*
     if (n == 0) return ISO_OK;
     const size_t smem = iso::mlp_smem();
     cudaFuncSetAttribute(iso::k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    iso::k_mlp_forward<<<iso::mlp_blocks(n, iso::device_sms()), 256, smem, static_cast<cudaStream_t>(stream)>>>(
+    iso::k_mlp_forward<<<iso::mlp_blocks(n, iso::device_sms(), 4), iso::kMlpThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         params, stats, isovals, n, y);
     return launch_status(cudaGetLastError());
 }
@@ -538,7 +646,7 @@ iso_status iso_mlp_predict(const float* params, int64_t n_sets, const iso_block_
         }
         ps.start[ps.n] = at;
         if (at == 0) continue;
-        iso::k_mlp_predict<<<iso::mlp_blocks(at, nsm), 256, smem, s>>>(params, ps, totals + s0);
+        iso::k_mlp_predict<<<iso::mlp_blocks(at, nsm, 4), iso::kMlpThreads, smem, s>>>(params, ps, totals + s0);
         if (cudaGetLastError() != cudaSuccess) return ISO_ERR_CUDA;
     }
     return ISO_OK;
@@ -552,10 +660,12 @@ iso_status iso_mlp_gradient(const float* params, const float* stats, const float
     if (cudaMemsetAsync(grads, 0, sizeof(float) * ISO_MLP_PARAMS, s) != cudaSuccess ||
         cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess)
         return ISO_ERR_CUDA;
-    const size_t smem = iso::mlp_smem();
+    const size_t smem = sizeof(iso::MlpGradSmem);
     cudaFuncSetAttribute(iso::k_mlp_gradient, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    iso::k_mlp_gradient<<<iso::mlp_blocks(n, iso::device_sms()), 256, smem, s>>>(params, stats, isovals, target, n,
-                                                                                grads, loss);
+    // whole clusters; a CTA without a tile adds zeros
+    const int blocks = (iso::mlp_blocks(n, iso::device_sms(), 2) + iso::kMlpCluster - 1) / iso::kMlpCluster *
+                       iso::kMlpCluster;
+    iso::k_mlp_gradient<<<blocks, iso::kMlpThreads, smem, s>>>(params, stats, isovals, target, n, grads, loss);
     return launch_status(cudaGetLastError());
 }
 
