@@ -115,6 +115,7 @@ SIGNATURES = {
     "iso_vtk_read_image": (C.c_int, [C.c_char_p, C.POINTER(IsoGrid), C.c_void_p]),
     "iso_vtk_write_mesh": (C.c_int, [C.c_char_p, C.POINTER(IsoMesh)]),
     "iso_vtk_write_image": (C.c_int, [C.c_char_p, C.POINTER(IsoGrid), C.c_void_p]),
+    "iso_populate_host": (C.c_int, [C.c_int64, C.POINTER(C.c_void_p), C.POINTER(C.c_int64)]),
     "iso_generate_blobs": (C.c_int, [C.POINTER(C.c_int64), C.c_int, C.c_uint64, C.c_void_p]),
     "iso_generate_value_noise": (C.c_int, [C.POINTER(C.c_int64), C.c_int, C.c_int, C.c_uint64, C.c_void_p]),
 }
