@@ -7,174 +7,141 @@
 // integers the conversion is exact, and for an integer s and a real iso,
 // s >= iso exactly when s >= ceil(iso); so the kernel compares the integer
 // sample with thr = ceil(iso) (clamped to the int range; a NaN isovalue, for
-// which every comparison is false, gives INT_MAX).  The bit words, counts and
-// row layout are those of k_count_tma (count_kernels.cu), so the scan and the
-// generate pass that follow are unchanged; the vertex pass reads the same
-// narrow samples (k_vertices with a sample type, vertices.cuh).
-//
-// k_count_narrow is k_count_tma for rows of up to 16 words whose byte length is
-// a multiple of 16 (the volume at a 16-byte boundary): a warp's rows jw ..
-// jw+RPW of a plane come into its shared buffer by one TMA bulk copy (bounded
-// mbarrier wait), plane k+2 in flight while plane k is counted; each lane
-// builds its own 32-point word from the buffer.
+// which every comparison is false, gives INT_MAX).  The rows, words and counts
+// are those of count_rows.cuh, so the scan and the generate pass that follow
+// are unchanged; the vertex pass reads the same narrow samples (k_vertices with
+// a sample type, vertices.cuh).
 #include <climits>
 #include <cmath>
 #include <cstdint>
 #include <type_traits>
 
 #include "../../include/miniiso.h"
-#include "count_words.cuh"
+#include "count_rows.cuh"
 #include "iso_kernels.h"
 
 namespace iso {
 
-// Bit i of the result: sample i of the 16-byte chunk v >= thr.
-template <typename S>
-__device__ __forceinline__ uint32_t chunk_bits(uint4 v, int thr)
-{
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    uint32_t b = 0u;
+// Two or four samples of a 32-bit word compared at once.  With a sample's top
+// bit set and the threshold's cleared, their difference keeps its top bit
+// exactly when the low bits alone are at or above the threshold's, and borrows
+// from no neighbour; the top bits then decide by themselves or leave it to
+// that.  Signed samples are the unsigned ones with the top bit the other way
+// round.  1.35 (8 bits) and 2.6 (16 bits) instructions a sample, where a
+// compare, a select and a shift per sample took 4 to 5.
+template <typename S, bool ALIGNED>
+struct IntSamples {
+    typedef S T;
+    static constexpr bool kAligned = ALIGNED;
+    static constexpr int B = 8 * (int)sizeof(S);
+    static constexpr int PER = 16 / (int)sizeof(S);  // samples of a 16-byte chunk
+    static constexpr int NV = 2 * (int)sizeof(S);    // chunks of a word
+    static constexpr uint32_t kOne = B == 8 ? 0x01010101u : 0x00010001u, kTop = kOne << (B - 1);
+    uint32_t low, high;  // the threshold's low bits; all ones where its top bit is clear
+    uint32_t on;         // the top bits, none when no sample reaches the threshold
+    struct Lane {
+        int off[NV];
+        int rot;
+    };
+    __device__ __forceinline__ IntSamples(int thr)
+    {
+        const int least = std::is_signed<S>::value ? -(1 << (B - 1)) : 0;
+        const uint32_t t = thr <= least ? 0u : (uint32_t)thr - (uint32_t)least;  // as of unsigned samples
+        on = (thr > least && t >> B) ? 0u : kTop;
+        low = (t & ((1u << (B - 1)) - 1u)) * kOne;
+        high = (t >> (B - 1)) & 1u ? 0u : 0xffffffffu;
+    }
+    // Neighbouring lanes start at different chunks of their words, so that a quarter warp reads different banks.
+    __device__ __forceinline__ Lane lane(int lane, int first) const
+    {
+        Lane x;
+        x.rot = (lane / (8 / NV) - first / PER) & (NV - 1);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if constexpr (sizeof(S) == 2) {
-            const int lo = std::is_signed<S>::value ? (int)(int16_t)(w[q] & 0xffffu) : (int)(w[q] & 0xffffu);
-            const int hi = std::is_signed<S>::value ? ((int)w[q] >> 16) : (int)(w[q] >> 16);
-            b |= (uint32_t)(lo >= thr) << (2 * q);
-            b |= (uint32_t)(hi >= thr) << (2 * q + 1);
+        for (int u = 0; u < NV; ++u) x.off[u] = ((u + x.rot) & (NV - 1)) * 16;
+        return x;
+    }
+    // the top bit of every sample of w: sample >= threshold
+    __device__ __forceinline__ uint32_t ge(uint32_t w) const
+    {
+        const uint32_t d = (w | kTop) - low;
+        const uint32_t u = std::is_signed<S>::value ? ~w : w;
+        return ((u & d) | ((u | d) & high)) & on;
+    }
+    // Bits of two chunks, the first sample in the lowest (8-bit samples: 32 bits; 16-bit: 16).
+    __device__ __forceinline__ uint32_t bits2(uint4 a, uint4 b) const
+    {
+        if constexpr (B == 8) {
+            // two words to a nibble pair per byte, whose bits 3 and 7 a multiplication brings next to the other
+            // bytes' in the top byte (no two of its terms meet)
+            constexpr uint32_t gather = 1u << 21 | 1u << 14 | 1u << 7 | 1u;
+            const uint32_t p0 = (ge(a.x) >> 4 | ge(a.y)) * gather, p1 = (ge(a.z) >> 4 | ge(a.w)) * gather;
+            const uint32_t p2 = (ge(b.x) >> 4 | ge(b.y)) * gather, p3 = (ge(b.z) >> 4 | ge(b.w)) * gather;
+            return __byte_perm(__byte_perm(p0, p1, 0x0073), __byte_perm(p2, p3, 0x0073), 0x5410);
         } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const uint32_t u = (w[q] >> (8 * e)) & 0xffu;
-                const int s = std::is_signed<S>::value ? (int)(int8_t)u : (int)u;
-                b |= (uint32_t)(s >= thr) << (4 * q + e);
-            }
+            // every second bit of both halves: odd samples above, even ones below
+            uint32_t r = ge(a.x);
+            r = r >> 2 | ge(a.y);
+            r = r >> 2 | ge(a.z);
+            r = r >> 2 | ge(a.w);
+            r = r >> 2 | ge(b.x);
+            r = r >> 2 | ge(b.y);
+            r = r >> 2 | ge(b.z);
+            r = r >> 2 | ge(b.w);
+            return r;
         }
     }
-    return b;
-}
+    // Word at sample index `at` of the buffer (row start + 32 * word); bits past the row are garbage.  Every lane of
+    // the warp calls it.  last: the lane's word is the row's last, nv its points inside the row.
+    __device__ __forceinline__ uint32_t word(const unsigned char* buf, int at, const Lane& x, bool last, int nv) const
+    {
+        const unsigned char* p = buf + 16 * (at / PER);
+        uint32_t w;
+        const uint32_t a = bits2(*reinterpret_cast<const uint4*>(p + x.off[0]),
+                                 *reinterpret_cast<const uint4*>(p + x.off[1]));
+        if constexpr (B == 8) {
+            w = a;
+        } else {
+            const uint32_t b = bits2(*reinterpret_cast<const uint4*>(p + x.off[2]),
+                                     *reinterpret_cast<const uint4*>(p + x.off[3]));
+            w = __byte_perm(a, b, 0x7632) | __byte_perm(a, b, 0x5410) >> 1;
+        }
+        w = __funnelshift_l(w, w, PER * x.rot);
+        if (ALIGNED) return w;
+        // the row starts at % PER samples into its first chunk: the points shifted out come from the next lane's
+        // word, or from one more chunk
+        const int sh = at & (PER - 1);
+        uint32_t hi = __shfl_down_sync(0xffffffffu, w, 1);
+        if (last && nv + sh > 32) {
+            const uint32_t c = bits2(*reinterpret_cast<const uint4*>(p + 16 * NV), make_uint4(0u, 0u, 0u, 0u));
+            // 16-bit samples: the chunk's bits went eight places further down, past the zeros' ones
+            hi = B == 8 ? c : (c >> 16 & 0xaau) | (c >> 1 & 0x55u);
+        }
+        return __funnelshift_r(w, hi, sh);
+    }
+};
 
-// Word wd (samples 32*wd .. 32*wd+31) of a row of nx samples in shared
-// memory, built by one lane: NV chunks of 16 bytes, read starting at chunk rot
-// so that neighbouring lanes read different bank groups, rotated into place at
-// the end.  FULL: every lane's word lies inside the row.
-template <typename S, bool FULL>
-__device__ __forceinline__ uint32_t row_word_n(const S* row, int nx, int wd, int rot, int thr)
+// R rows per lane by count_rows_plan's rule, which suits these samples too (times of any R above one and of half to
+// four times its planes per item lie within 5%).  The ALU pipe bounds it: 512 x 512 x 320 int16 52 us (66 with a
+// compare per sample and rows at powers of two of lanes; its bytes take 26), int8 39 (65).  Rows of 17-32 words and
+// rows that are not a multiple of 16 bytes come here too instead of through a float32 copy of the volume: extraction
+// of 667 x 328 x 324 int16 254 us against 464, 301 x 417 x 290 uint8 141 against 246.
+template <bool MC, typename S, int R, bool ALIGNED>
+__global__ void __launch_bounds__(kCountThreads) k_count_narrow(const S* __restrict__ vol, Grid g, int thr, int KC,
+                                                                int ngroups, unsigned nitems, int stage_bytes,
+                                                                uint4* __restrict__ rowcnt,
+                                                                uint32_t* __restrict__ mccnt,
+                                                                uint32_t* __restrict__ bits_out,
+                                                                unsigned long long* __restrict__ status)
 {
-    constexpr int PER = 16 / (int)sizeof(S);  // samples per chunk
-    constexpr int NV = 32 / PER;              // chunks per word
-    const uint4* r = reinterpret_cast<const uint4*>(row + 32 * wd);
-    const int nvalid = FULL ? NV : (nx - 32 * wd) / PER;  // nx is a multiple of PER
-    uint32_t w = 0u;
-#pragma unroll
-    for (int u = 0; u < NV; ++u) {
-        const int q = (u + rot) & (NV - 1);
-        if (FULL || q < nvalid) w |= chunk_bits<S>(r[q], thr) << (PER * u);
-    }
-    return NV == 1 ? w : __funnelshift_l(w, w, PER * rot);
-}
-
-template <bool MC, typename S, int RPW, bool FULL>
-__global__ void __launch_bounds__(kThreads, 4) k_count_narrow(const S* __restrict__ vol, Grid g, int thr, int KC,
-                                                           int nyb, uint4* __restrict__ rowcnt,
-                                                           uint32_t* __restrict__ mccnt, uint32_t* __restrict__ bits_out,
-                                                           unsigned long long* __restrict__ status)
-{
-    constexpr int LPR = 32 / RPW, NBUF = RPW + 1;
-    constexpr int NV = 2 * (int)sizeof(S);  // 16-byte chunks per 32-point word
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ uint64_t s_bar[kCountRows];
-    const int jb = blockIdx.x % nyb, kc = blockIdx.x / nyb;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane / LPR, lw = lane % LPR;
-    const int jw = jb * kCountRows * RPW + RPW * warp;
-    if (jw >= g.ny) return;  // all the warp's rows past the grid
-    S* buf = reinterpret_cast<S*>(s_raw) + (size_t)warp * NBUF * g.nx;
-    uint64_t* bar = &s_bar[warp];
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    const int j = jw + h;
-    const bool row_ok = j < g.ny;
-    const int kb = g.kr + kc * KC, ke = min(kb + KC, g.ke);
-    const bool hasY = row_ok && j < g.ny - 1;
-    const int nrows = min(NBUF, g.ny - jw);
-    const unsigned bytes = (unsigned)(nrows * g.nx * (int)sizeof(S));
-    const int rot = lane & (NV - 1);
-
-    auto issue = [&](int p) {
-        if (lane == 0) {
-            fence_proxy_async();
-            mbar_arrive_expect_tx(bar, bytes);
-            bulk_copy_g2s(buf, vol + ((long long)(p - g.kd) * g.ny + jw) * g.nx, bytes, bar);
-        }
-    };
-    unsigned phase = 0;
-    auto take = [&](uint32_t& wa, uint32_t& wb) -> bool {
-        __syncwarp();
-        const bool done = mbar_wait(bar, phase);
-        if (!__all_sync(0xffffffffu, done)) return false;
-        phase ^= 1u;
-        wa = row_ok ? row_word_n<S, FULL>(buf + h * g.nx, g.nx, lw, rot, thr) : 0u;
-        wb = hasY ? row_word_n<S, FULL>(buf + (h + 1) * g.nx, g.nx, lw, rot, thr) : 0u;
-        __syncwarp();  // every lane has read the buffer before it is refilled
-        return true;
-    };
-    // per-row totals: rows 2p, 2p+1 of the warp in the two 16-bit halves of reduction p
-    auto row_sum = [&](uint32_t v) -> uint32_t {
-        const int sh = 16 * (h & 1);
-        uint32_t mine = 0u;
-#pragma unroll
-        for (int p = 0; p < RPW / 2; ++p) {
-            const uint32_t s = __reduce_add_sync(0xffffffffu, (h >> 1) == p ? v << sh : 0u);
-            if ((h >> 1) == p) mine = s;
-        }
-        return (mine >> sh) & 0xffffu;
-    };
-
-    uint32_t A = 0, B = 0, Cw = 0, Dw = 0;
-    bool ok = true;
-    issue(kb);
-    ok = take(A, B);
-    if (ok && kb + 1 < g.nz) issue(kb + 1);
-    for (int k = kb; ok && k < ke; ++k) {
-        const bool hasZ = k + 1 < g.nz;
-        Cw = Dw = 0u;
-        if (hasZ) {  // plane k+1 was issued one step earlier
-            if (!(ok = take(Cw, Dw))) break;
-            if (k + 2 < g.nz && k + 1 < ke) issue(k + 2);
-        }
-        RowCounts rc;
-        RowWords rw;
-        rw.a = A;
-        rw.b = B;
-        rw.c = Cw;
-        rw.d = Dw;
-        const uint32_t an = __shfl_down_sync(0xffffffffu, rw.a, 1, LPR);
-        const uint32_t bn = __shfl_down_sync(0xffffffffu, rw.b, 1, LPR);
-        const uint32_t cn = __shfl_down_sync(0xffffffffu, rw.c, 1, LPR);
-        const uint32_t dn = __shfl_down_sync(0xffffffffu, rw.d, 1, LPR);
-        const bool nxt = lw < LPR - 1;
-        rw.ash = (rw.a >> 1) | ((nxt ? an : 0u) << 31);
-        rw.bsh = (rw.b >> 1) | ((nxt ? bn : 0u) << 31);
-        rw.csh = (rw.c >> 1) | ((nxt ? cn : 0u) << 31);
-        rw.dsh = (rw.d >> 1) | ((nxt ? dn : 0u) << 31);
-        if (row_ok) count_word<MC>(rw, lw, g, j, k, hasY, hasZ, false, rc);
-        const long long r = (long long)(k - g.kr) * g.ny + j;
-        if (row_ok && lw < g.W) bits_out[r * g.W + lw] = rw.a;
-        const uint32_t sx = row_sum(rc.xc), sy = row_sum(rc.yc), sz = row_sum(rc.zc), st = row_sum(rc.tc);
-        const uint32_t sm = MC ? row_sum(rc.mc) : 0u;
-        if (row_ok && lw == 0) {
-            rowcnt[r] = make_uint4(sx, sy, sz, st);
-            if (MC) mccnt[r] = sm;
-        }
-        A = Cw;
-        B = Dw;
-    }
-    if (!ok) {  // a copy did not complete in time: report it, and let the copy land before the CTA ends
-        if (lane == 0) atomicOr(status, kStatusTimeout);
-        mbar_wait(bar, phase);
-    }
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ uint64_t s_bar[kCountWarps];
+    next_may_start();
+    const int warp = threadIdx.x >> 5;
+    const unsigned item = blockIdx.x * kCountWarps + warp;
+    if (item >= nitems) return;
+    const IntSamples<S, ALIGNED> smp(thr);
+    count_rows_item<IntSamples<S, ALIGNED>, MC, R>(vol, g, smp, KC, ngroups, item, s_raw + (size_t)warp * stage_bytes,
+                                                   s_bar + warp, rowcnt, nullptr, mccnt, bits_out, status);
 }
 
 int narrow_threshold(float iso)
@@ -189,33 +156,23 @@ int narrow_threshold(float iso)
 bool narrow_fits(const Grid& g, const void* vol, int dtype)
 {
     const size_t sb = dtype_bytes(dtype);
-    return (sb == 1 || sb == 2) && g.kd == 0 && g.kr == 0 && g.ke == g.nz && g.W <= 16 &&
-           ((size_t)g.nx * sb) % 16 == 0 && (reinterpret_cast<uintptr_t>(vol) & 15) == 0;
+    return (sb == 1 || sb == 2) && g.kd == 0 && g.kr == 0 && g.ke == g.nz && g.W <= 32 &&
+           (reinterpret_cast<uintptr_t>(vol) & 15) == 0;
 }
 
 template <bool MC, typename S>
 static void narrow_launch(const CountPlan& p, const S* vol, const Grid& g, int thr, FeBuffers& b, cudaStream_t s)
 {
-    const int rpw = g.W <= 4 ? 8 : (g.W <= 8 ? 4 : 2);
-    const int rows = kCountRows * rpw;
-    const int nyb = (g.ny + rows - 1) / rows;
-    const unsigned blocks = (unsigned)(nyb * p.nkc);
-    const size_t smem = (size_t)kCountRows * (rpw + 1) * g.nx * sizeof(S);
-    const bool full = g.nx == 32 * (32 / rpw);
-#define ISO_NARROW(RPW, FULL)                                                                               \
-    {                                                                                                       \
-        auto kern = k_count_narrow<MC, S, RPW, FULL>;                                                      \
-        allow_smem(kern, smem);                                                                             \
-        kern<<<blocks, kThreads, smem, s>>>(vol, g, thr, p.KC, nyb, b.rowcnt, b.mccnt, b.bits, b.totals + 3); \
-    }
-    if (rpw == 8) {
-        if (full) ISO_NARROW(8, true) else ISO_NARROW(8, false)
-    } else if (rpw == 4) {
-        if (full) ISO_NARROW(4, true) else ISO_NARROW(4, false)
-    } else {
-        if (full) ISO_NARROW(2, true) else ISO_NARROW(2, false)
-    }
-#undef ISO_NARROW
+    const bool aligned = g.nx * (int)sizeof(S) % 16 == 0;
+    const CountRows r = count_rows_plan(g, p.nsm, (int)sizeof(S), aligned, false);
+    const size_t smem = (size_t)kCountWarps * r.stage;
+    const unsigned nb = (r.items + kCountWarps - 1) / kCountWarps;
+    auto kern = r.S == 4 ? (aligned ? k_count_narrow<MC, S, 4, true> : k_count_narrow<MC, S, 4, false>)
+              : r.S == 2 ? (aligned ? k_count_narrow<MC, S, 2, true> : k_count_narrow<MC, S, 2, false>)
+                         : (aligned ? k_count_narrow<MC, S, 1, true> : k_count_narrow<MC, S, 1, false>);
+    allow_smem(kern, smem);
+    kern<<<nb, kCountThreads, smem, s>>>(vol, g, thr, r.KC, r.groups, r.items, r.stage, b.rowcnt, b.mccnt, b.bits,
+                                         b.totals + 3);
 }
 
 void launch_count_narrow(const void* vol, int dtype, const Grid& g, float iso, bool mc, const CountPlan& p, FeBuffers& b,

@@ -140,7 +140,7 @@ __device__ __forceinline__ uint32_t row_total(uint32_t v, int lw, int W)
 __host__ __device__ inline int count_stage_bytes(int nx, int W, int S, int sample_bytes, bool aligned)
 {
     const int rows = (32 / W) * S + 1;
-    return ((rows * nx + (aligned ? 0 : 3)) * sample_bytes + kCountPad + 15) & ~15;
+    return ((rows * nx + (aligned ? 0 : 16 / sample_bytes - 1)) * sample_bytes + kCountPad + 15) & ~15;
 }
 
 // Item `item` of a grid: row group item % ngroups, planes [kc * KC, ...) of
@@ -159,6 +159,7 @@ __device__ __forceinline__ void count_rows_item(const typename Samples::T* __res
 {
     typedef typename Samples::T T;
     constexpr bool ALIGNED = Samples::kAligned;
+    constexpr int PER = 16 / (int)sizeof(T);  // samples of 16 bytes
     const int lane = threadIdx.x & 31;
     const int W = g.W, rpw = 32 / W, G = rpw * S;
     const int grp = (int)(item % (unsigned)ngroups), kc = (int)(item / (unsigned)ngroups);
@@ -187,10 +188,10 @@ __device__ __forceinline__ void count_rows_item(const typename Samples::T* __res
     // point to the one at or above their last, except past the end of the pass' last plane, where the last points
     // come by plain loads.  points [s0, e) -> copied [a0, e1)
     auto extent = [&](long long s0, long long& a0, long long& e1) {
-        a0 = s0 & ~3ll;
+        a0 = s0 & ~(long long)(PER - 1);
         const long long e = s0 + (long long)nrows * g.nx;
-        e1 = (e + 3) & ~3ll;
-        if (e1 > (long long)(plast - g.kd + 1) * g.ny * g.nx) e1 = e & ~3ll;
+        e1 = (e + PER - 1) & ~(long long)(PER - 1);
+        if (e1 > (long long)(plast - g.kd + 1) * g.ny * g.nx) e1 = e & ~(long long)(PER - 1);
         return e;
     };
     auto issue = [&](int p) {  // lane 0; the buffer's readers were joined by a __syncwarp
