@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(kThreads, vertex_ctas_per_sm(MC))
                const unsigned long long* __restrict__ starts, const unsigned long long* __restrict__ totals,
                long long capV, long long capT, float* __restrict__ points, float* __restrict__ normals)
 {
+    wait_for_previous();
     next_may_start();
     if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
     auto first = [&](int p) { return p < g.ke ? starts[COMP * g.R + (long long)(p - g.kr) * g.ny] : totals[COMP]; };
@@ -156,10 +157,16 @@ inline void launch_vertices_impl(const S* vol, const Grid& g, float iso, const F
     // one wave, or fewer CTAs when the mesh cannot hold that many vertices (small grids in a batch)
     const long long wave = (long long)nsm * vertex_ctas_per_sm(MC);
     const unsigned blocks = (unsigned)std::min(wave, (capV + kThreads - 1) / kThreads);
-    // an ordinary launch: brought in beside the end of the generate kernel, whose shared memory leaves an SM little L1,
-    // it would keep that split to its end, and the gathers live on the L1 (512^3: the call 622 us instead of 376)
-    k_vertices<MC, COMP, S><<<blocks, kThreads, 0, s>>>(vol, g, make_grad_scale(g), iso, k0, k1, b.starts, b.totals, capV,
-                                               capT, points, normals);
+    // Brought in beside the end of the generate kernel, whose shared memory leaves an SM little L1, it keeps that split
+    // to its end, and on large grids the gathers live on the L1 (512^3: the call 622 us instead of 376; 384^3 noise 229
+    // for 201, 200^3 72.5 for 70.4). Up to 2^22 points the earlier start is worth more (64^3 50 us -> 48, 160^3 63.8 ->
+    // 62.5, blobs 59.6 -> 58.9).
+    if ((long long)g.nx * g.ny * (g.ke - g.kr) <= 1ll << 22)
+        launch_after(k_vertices<MC, COMP, S>, blocks, kThreads, 0, s, vol, g, make_grad_scale(g), iso, k0, k1, b.starts,
+                     b.totals, capV, capT, points, normals);
+    else
+        k_vertices<MC, COMP, S><<<blocks, kThreads, 0, s>>>(vol, g, make_grad_scale(g), iso, k0, k1, b.starts, b.totals,
+                                                            capV, capT, points, normals);
 }
 
 }  // namespace iso
