@@ -147,6 +147,12 @@ inline void build_case_tables(CaseTables& t)
             }
             t.corner[5 * m + q] = x;
         }
+        uint32_t own = 0, nown = 0;  // edges that a cell away from the first column, row and plane owns (mc_owned_edges)
+        for (int q = 0; q < iso_case_ntris(t.order[c]); ++q) {
+            const int e = iso_case_edge(t.order[c], q);
+            if (e == 5 || e == 6 || e == 11) own |= (uint32_t)e << (8 + 4 * nown++);
+        }
+        t.own2[m] = own | nown;
         uint32_t places = 0;
         for (int b = 0, n = 0; b < 8; ++b)
             if ((m >> b) & 1) places |= (uint32_t)b << (4 * n++);

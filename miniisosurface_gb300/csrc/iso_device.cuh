@@ -50,6 +50,7 @@ struct CaseTables {
                                // (axis * 16 + next row * 48 + next plane * 8, bit 0: the edge at point i + 1)
     uint32_t nth[256];     // of a byte: the places of its set bits, a nibble each
     uint64_t order2[256];
+    uint32_t own2[256];    // MC: count | edges << 8, 12, 16 that an inner cell owns, in order of appearance
     uint16_t cut2[256];
     uint8_t nt2[256];      // triangles of the case
 };
