@@ -7,8 +7,8 @@
 // KC planes -- from a counter and marches along z on its own.  A row's W words
 // go to W neighbouring lanes, rpw rows side by side (32 / W of them; fewer on
 // grids with too few rows for the GPU), and a lane holds kGenSlots rows (slot
-// s: row jw + s * rpw + lane / W), the last slot the row after the group: the
-// fixed work of a step is shared by up to 64 words, and their active cells and
+// s: row jw + s * rpw + lane / W), the last row, or one in a slot more, the row
+// after the group: the fixed work of a step is shared by up to 64 words, and their active cells and
 // triangles fill batches of 32 lanes (one row pair at a time left a third of the
 // lanes idle).
 //
@@ -17,7 +17,7 @@
 // cell row that touches it: the warp keeps {mask, id of its first cut edge} of
 // x, y and z of every word and row in shared memory, the planes' two copies
 // side by side, and a triangle corner is one 8-byte load and a popc:
-//   tab[idx][axis][plane & 1]   48 bytes per word, idx = w * (G + 1) + row, G + 1
+//   tab[idx][axis][plane & 1]   48 bytes per word, idx = w * (2 * rpw + 1) + row,
 //                               odd so that neighbouring words fall on different banks
 //   pair[idx][plane & 1]        {word, next word} of the row
 // With that order the word above in y is 48 bytes on at any width, so a corner
@@ -27,8 +27,8 @@
 // What bounds it: instruction issue (77% of the slots on the 512^3 volume, with 117 M warp instructions; the kernels
 // it replaced, which recomputed eight masks and four scans per row and step, took 161 M).  Events around the pass, us,
 // Flying Edges, before / now: 512^3 167 / 128, 768^3 (with the vertices, which were in the same kernel) 1252 / 722,
-// 667 x 228 x 724 the same 363 / 208, 150 x 700 x 600 110 / 77, 301 x 217 x 190 36 / 30, 128^3 22 / 19, 64^3 17 / 15.
-// Three rows per lane instead of two: 145 us at 512^3 (fewer warps fit).  Vertex runs made dense like the cells
+// 667 x 228 x 724 the same 363 / 208, 150 x 700 x 600 110 / 70, 301 x 217 x 190 36 / 28, 128^3 22 / 16.6, 64^3 17 / 13.3.
+// Three rows per lane and one more instead of two and one: 145 us at 512^3 (fewer warps fit).  Vertex runs made dense like the cells
 // instead of a loop over each word's bits: 32 M instructions instead of 21 M.
 // Marching Cubes: a cell away from the first column, row and plane owns at most three vertices, read ready from a
 // table instead of walking the case's edges one by one, and a chunk's vertices are written together: 512^3 187 us
@@ -40,12 +40,17 @@
 
 namespace iso {
 
-constexpr int kGenSlots = 2;       // rows per lane; the row after the group takes one more slot
+constexpr int kGenSlots = 2;       // rows per lane
+constexpr int kGenExtra = 2;       // rows side by side up to which a kernel for them gives the row after the group a slot
 constexpr int kGenChunk = 64;      // cells whose triangles are listed together
 constexpr int kGenMaxWarps = 16;   // warps per CTA, two CTAs per SM
 
-// Rows held by a warp: the group's and the one after it.
-__host__ __device__ inline int gen_held_rows(int rpw) { return kGenSlots * rpw + 1; }
+// Rows held by a warp: the group's and the one after it, which takes a slot of its own (extra) or is the last of the
+// slots' rows.
+__host__ __device__ inline constexpr bool gen_extra_slot(int RPW) { return RPW > 0 && RPW <= kGenExtra; }
+__host__ __device__ inline constexpr int gen_group_rows(int rpw, bool extra) { return kGenSlots * rpw - (extra ? 0 : 1); }
+// Entries of a word in the warp's tables: odd, so that neighbouring words fall on different banks.
+__host__ __device__ inline int gen_word_entries(int rpw) { return kGenSlots * rpw + 1; }
 
 // Per-warp scratch: tab, pair, cell[chunk], the triangle list (u16), and for the Marching Cubes modes the
 // cells' places and the owned vertices' list.
@@ -55,7 +60,7 @@ __host__ __device__ inline int gen_cells_scratch(int W, int rpw, int mode)
     const int list = mode == kGenMC ? 0 : 5 * kGenChunk * 2;
     const int own = gen_owns(mode) ? 4 * kGenChunk + 2 * kGenOwned : 0;
     // + 48: the last row of a slot looks one entry past its word's rows
-    return (64 * W * gen_held_rows(rpw) + 48 + 4 * kGenChunk + list + own + 15) & ~15;
+    return (64 * W * gen_word_entries(rpw) + 48 + 4 * kGenChunk + list + own + 15) & ~15;
 }
 
 // The kernel's per-case tables in shared memory (CaseTables holds them ready).
@@ -137,14 +142,14 @@ struct GenLane {
     uint32_t evalid;   // x-edges / cells of its word: i <= nx-2
 };
 
-__device__ __forceinline__ GenLane gen_lane(const Grid& g, int rpw)
+__device__ __forceinline__ GenLane gen_lane(const Grid& g, int rpw, bool extra)
 {
     GenLane l;
-    const int lane = threadIdx.x & 31, G1 = gen_held_rows(rpw);
+    const int lane = threadIdx.x & 31;
     l.h = lane / g.W;
     l.lw = lane - l.h * g.W;
-    l.idx0 = l.lw * G1 + l.h;
-    l.rows = l.h < rpw ? G1 - l.h : 0;
+    l.idx0 = l.lw * gen_word_entries(rpw) + l.h;
+    l.rows = l.h < rpw ? gen_group_rows(rpw, extra) + 1 - l.h : 0;
     l.evalid = validmask(l.lw, g.nx - 1);
     return l;
 }
@@ -161,15 +166,15 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
 {
     constexpr bool OWNS = GenCellTables<MODE>::OWNS, TRIS = GenCellTables<MODE>::TRIS;
     constexpr bool WIDE = MODE == kGenFE && sizeof(IndexT) == 8;  // ids past 32 bits; the map's ids are 32-bit
-    constexpr int S = kGenSlots, NS = S + 1;
+    constexpr int S = kGenSlots, NS = S + (gen_extra_slot(RPW) ? 1 : 0);
     static_assert(S == 2, "the active cells' counts of a lane's slots share a word");
     const int rpw = RPW > 0 ? RPW : rpw_;
     const int lane = threadIdx.x & 31;
-    const int W = g.W, RW = rpw * W, G1 = gen_held_rows(rpw), G = G1 - 1;
+    const int W = g.W, RW = rpw * W, E = gen_word_entries(rpw), G = gen_group_rows(rpw, gen_extra_slot(RPW));
     const int h = ln.h, lw = ln.lw, idx0 = ln.idx0;
     unsigned char* tab = s_raw + ws;
-    unsigned char* pair = tab + 48 * W * G1;
-    uint32_t* cell = reinterpret_cast<uint32_t*>(pair + 16 * W * G1 + 48);
+    unsigned char* pair = tab + 48 * W * E;
+    uint32_t* cell = reinterpret_cast<uint32_t*>(pair + 16 * W * E + 48);
     uint16_t* list = reinterpret_cast<uint16_t*>(cell + kGenChunk);
     uint32_t* place = reinterpret_cast<uint32_t*>(list + (TRIS ? 5 * kGenChunk : 0));
     uint16_t* vlist = reinterpret_cast<uint16_t*>(place + kGenChunk);
@@ -251,7 +256,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                         if (s < S) *reinterpret_cast<uint2*>(t + 16 + par) = make_uint2(y[s], yf);
                         *reinterpret_cast<uint2*>(t + 32 + kpar) = make_uint2(z[s], zf);
                     }
-                    if (MODE == kGenFE && s < S && s * rpw < ln.rows) {  // vertex records of the word's cut edges
+                    if (MODE == kGenFE && s < S && s * rpw < ln.rows - 1) {  // vertex records of the word's cut edges
                         const uint32_t j = (uint32_t)(jw + s * rpw + h);
                         auto records = [&](uint32_t mk, uint32_t first, unsigned long long row0, uint32_t axis, uint32_t k) {
                             const unsigned long long at = WIDE ? row0 - vbase + (uint32_t)(first - (uint32_t)row0)
@@ -334,7 +339,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                         cell[cb + lane] = (48u * id) | ((uint32_t)b << 13) | ((5u * cs) << 18);
                         if (TRIS) nt = tabs.nt[cs];
                         if (OWNS) {
-                            row = id - (uint32_t)(slw * G1);
+                            row = id - (uint32_t)(slw * E);
                             place[cb + lane] = (uint32_t)(32 * slw + b) | (row << 10);
                         }
                     }
@@ -456,7 +461,7 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells(
     // with the same masks; the writes are not checked one by one.
     if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
     const uint32_t ws = (threadIdx.x >> 5) * (uint32_t)ws_bytes;
-    const GenLane ln = gen_lane(g, RPW > 0 ? RPW : rpw);
+    const GenLane ln = gen_lane(g, RPW > 0 ? RPW : rpw, gen_extra_slot(RPW));
     for (uint32_t item; (item = gen_take(work)) < nitems;) {
         gen_cells_item<IndexT, MODE, RPW>(item, s_raw, ws, tabs, bits, g, ln, rpw, cols, ngroups, kbeg, kend, kemit,
                                           vbase, tbase, row4, rs, points, tris, fe2mc, reverse);
@@ -488,7 +493,7 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells_batch(
         rs.ny = g.ny;
         rs.kr = g.kr;
         rs.add[0] = rs.add[1] = rs.add[2] = rs.add[3] = 0;
-        gen_cells_item<IndexT, kGenFE, 0>(item - __ldg(&first[q]), s_raw, ws, tabs, d->bits, g, gen_lane(g, 32 / g.W),
+        gen_cells_item<IndexT, kGenFE, 0>(item - __ldg(&first[q]), s_raw, ws, tabs, d->bits, g, gen_lane(g, 32 / g.W, false),
                                        32 / g.W, GenCols{0, 1, d->gen_KC}, d->gen_ngroups, g.kr, g.ke, g.kr, 0ull, 0ull, d->row4, rs,
                                        d->points, static_cast<IndexT*>(d->tris), nullptr, reverse);
     }
@@ -511,13 +516,18 @@ void launch_gen_cells(const Grid& g, const CaseTables* cases, const FeBuffers& b
     const int nzw = p.kend - p.kbeg;
     if (nzw <= 0) return;
     // Rows side by side: all that fit, halved on grids whose (row group, plane) steps would not fill three quarters
-    // of a wave (128^3: 18.2 us with two against 19.7 with eight; 256^3, filled: 34 with four, 39 with two).
-    int rpw = 32 / g.W, per_cta;
+    // of a wave (128^3: 18.2 us with two against 19.7 with eight; 256^3, filled: 34 with four, 39 with two). The row
+    // after the group in a slot of its own (three slots of work for a group of twice rpw rows, against two for one row
+    // less) only where one or two rows are all that fit: 512^3 126 us against 131, but 256^3 33.7 against 31.3 without
+    // it, 150 x 700 x 600 75.5 / 70, 128^3 17.5 / 16.6.
+    int rpw = 32 / g.W, per_cta, rows;
+    bool extra = gen_extra_slot(rpw);
     long long ngroups, wave;
-    for (;; rpw /= 2) {
+    for (;; rpw /= 2, extra = false) {
         per_cta = gen_cells_warps(gen_cells_scratch(g.W, rpw, MODE), sizeof(GenCellTables<MODE>));
         wave = 2ll * p.nsm * per_cta;
-        ngroups = (g.ny + kGenSlots * rpw - 1) / (kGenSlots * rpw);
+        rows = gen_group_rows(rpw, extra);
+        ngroups = (g.ny + rows - 1) / rows;
         if (rpw <= 3 || 4 * ngroups * nzw >= 3 * wave) break;
     }
     const int ws_bytes = gen_cells_scratch(g.W, rpw, MODE);
@@ -539,7 +549,7 @@ void launch_gen_cells(const Grid& g, const CaseTables* cases, const FeBuffers& b
     unsigned int* work = reinterpret_cast<unsigned int*>(b.totals + 7);
     if (again) cudaMemsetAsync(work, 0, sizeof(unsigned int), s);
     const size_t smem = (size_t)warps * ws_bytes;
-    auto kern = rpw == 1 ? k_gen_cells<IndexT, MODE, 1> : (rpw == 2 ? k_gen_cells<IndexT, MODE, 2> : k_gen_cells<IndexT, MODE, 0>);
+    auto kern = !extra ? k_gen_cells<IndexT, MODE, 0> : (rpw == 1 ? k_gen_cells<IndexT, MODE, 1> : k_gen_cells<IndexT, MODE, 2>);
     allow_smem(kern, smem);
     launch_after(kern, (unsigned)blocks, 32u * warps, smem, s, b.bits, g, rpw, cols, (int)ngroups, (uint32_t)nitems,
                  p.kbeg, p.kend, p.kemit, p.vbase, p.tbase, ws_bytes, cases, b.row4, rs, b.totals, work, capV, capT,

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, vertex_ctas_per_sm(false))
 
 int gen_batch_ws_bytes(int W) { return gen_cells_scratch(W, 32 / W, kGenFE); }
 
-int gen_batch_rows(int W) { return gen_held_rows(32 / W) - 1; }
+int gen_batch_rows(int W) { return gen_group_rows(32 / W, false); }
 
 void launch_gen_batch(int index_bytes, const BatchReq* reqs, const int* list, const unsigned* first, int m,
                       unsigned nitems, const CaseTables* cases, unsigned* work, int ws_bytes, int reverse, int nsm,
