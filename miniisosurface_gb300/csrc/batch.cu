@@ -93,7 +93,7 @@ bool fusable(const iso_ctx* ctx, const iso_request& r, const BatchItem& it)
 // Work split of the fused launches: count blocks of at least kc planes, generate items for about ipw per warp
 // of one wave (the autotuner's candidates; 0: the defaults).
 constexpr int kFusedKC[] = {8, 16, 32};
-constexpr int kFusedIPW[] = {8, 16, 32};
+constexpr int kFusedIPW[] = {16, 32, 64};
 constexpr int kFusedKCDefault = 16, kFusedIPWDefault = 16;
 
 FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, std::vector<BatchItem>& items,
