@@ -44,6 +44,9 @@ constexpr int kGenSlots = 2;       // rows per lane
 constexpr int kGenExtra = 2;       // rows side by side up to which a kernel for them gives the row after the group a slot
 constexpr int kGenChunk = 64;      // cells whose triangles are listed together
 constexpr int kGenMaxWarps = 16;   // warps per CTA, two CTAs per SM
+// ... of the batch kernel, which holds what others take from their parameters in registers: with 16 it spilled 29 of
+// them (64 uneven volumes, whole call 2030 us; 14: 1960, 12: 1970, 10: 2013)
+constexpr int kGenBatchWarps = 14;
 
 // Rows held by a warp: the group's and the one after it, which takes a slot of its own (extra) or is the last of the
 // slots' rows.
@@ -154,15 +157,30 @@ __device__ __forceinline__ GenLane gen_lane(const Grid& g, int rpw, bool extra)
     return l;
 }
 
+// Where an item's records and triangles go: kernel parameters, or the request's copy in shared memory, read anew at
+// each use because the batch kernel has no registers left for it.
+template <typename IndexT>
+struct GenOut {
+    float* p;
+    IndexT* t;
+    __device__ __forceinline__ float* points() const { return p; }
+    __device__ __forceinline__ IndexT* tris() const { return t; }
+};
+template <typename IndexT>
+struct GenOutShared {
+    const volatile unsigned long long* s;
+    __device__ __forceinline__ float* points() const { return reinterpret_cast<float*>(s[0]); }
+    __device__ __forceinline__ IndexT* tris() const { return reinterpret_cast<IndexT*>(s[1]); }
+};
+
 // Work item `item` of an extraction, run by one warp with its scratch at s_raw + ws.
-template <typename IndexT, int MODE, int RPW>
+template <typename IndexT, int MODE, int RPW, typename Out>
 __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_raw, uint32_t ws,
                                                const GenCellTables<MODE>& tabs, const uint32_t* __restrict__ bits,
                                                const Grid& g, const GenLane& ln, int rpw_, const GenCols& cols, int ngroups,
                                                int kbeg, int kend, int kemit, unsigned long long vbase,
                                                unsigned long long tbase, const uint4* __restrict__ row4,
-                                               const RowStarts& rs, float* __restrict__ points,
-                                               IndexT* __restrict__ tris, uint32_t* __restrict__ fe2mc, int reverse)
+                                               const RowStarts& rs, const Out& out, uint32_t* __restrict__ fe2mc, int reverse)
 {
     constexpr bool OWNS = GenCellTables<MODE>::OWNS, TRIS = GenCellTables<MODE>::TRIS;
     constexpr bool WIDE = MODE == kGenFE && sizeof(IndexT) == 8;  // ids past 32 bits; the map's ids are 32-bit
@@ -261,7 +279,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                         auto records = [&](uint32_t mk, uint32_t first, unsigned long long row0, uint32_t axis, uint32_t k) {
                             const unsigned long long at = WIDE ? row0 - vbase + (uint32_t)(first - (uint32_t)row0)
                                                                : (unsigned long long)(uint32_t)(first - (uint32_t)vbase);
-                            float* o = points + 3 * at;
+                            float* o = out.points() + 3 * at;
                             while (mk != 0u) {
                                 put_vertex_record(o, 0ull, (uint32_t)(32 * lw + __ffs(mk) - 1), axis, j, k);
                                 mk &= mk - 1u;
@@ -389,7 +407,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                         int dx, dy, dz, axis;
                         cube_edge_geometry(e12, dx, dy, dz, axis);
                         if (k >= kemit)  // cell rows below kemit belong to the slab below: map only
-                            put_mc_record(points, mid - vbase, (pl & 1023u) + (uint32_t)dx, (uint32_t)axis,
+                            put_mc_record(out.points(), mid - vbase, (pl & 1023u) + (uint32_t)dx, (uint32_t)axis,
                                           (uint32_t)(dx | (dy << 1) | (dz << 2)), (uint32_t)(jw + dy) + (pl >> 10),
                                           (uint32_t)(k + dz));
                         // the edge's Flying Edges id: its axis, row and plane in tab, dx bits further along x
@@ -401,7 +419,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                     mcur += nown;
                 }
                 if (TRIS) {
-                    IndexT* o = tris + 3 * (tcur + (uint32_t)lane - tbase);
+                    IndexT* o = out.tris() + 3 * (tcur + (uint32_t)lane - tbase);
                     for (uint32_t t = (uint32_t)lane; t < ntri; t += 32, o += 96) {
                         const uint32_t c = list[t];
                         const uint32_t rec = cell[c & 63u];
@@ -464,19 +482,20 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells(
     const GenLane ln = gen_lane(g, RPW > 0 ? RPW : rpw, gen_extra_slot(RPW));
     for (uint32_t item; (item = gen_take(work)) < nitems;) {
         gen_cells_item<IndexT, MODE, RPW>(item, s_raw, ws, tabs, bits, g, ln, rpw, cols, ngroups, kbeg, kend, kemit,
-                                          vbase, tbase, row4, rs, points, tris, fe2mc, reverse);
+                                          vbase, tbase, row4, rs, GenOut<IndexT>{points, tris}, fe2mc, reverse);
     }
 }
 
 // The Flying Edges generate items of a list of requests (batch_kernels.cuh), one launch: item x is item
 // x - first[q] of request list[q]; the items of a request whose mesh cannot hold its counts are skipped.
 template <typename IndexT>
-__global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells_batch(
+__global__ void __launch_bounds__(32 * kGenBatchWarps, 2) k_gen_cells_batch(
     const BatchReq* __restrict__ reqs, const int* __restrict__ list, const unsigned* __restrict__ first, int m,
     const CaseTables* __restrict__ cases, unsigned int* __restrict__ work, int ws_bytes, int reverse)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ GenCellTables<kGenFE> tabs;
+    __shared__ unsigned long long s_out[kGenBatchWarps][2];
     stage_gen_tables<kGenFE>(cases, tabs);
     __syncthreads();
     const uint32_t ws = (threadIdx.x >> 5) * (uint32_t)ws_bytes;
@@ -487,6 +506,13 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells_batch(
         if ((long long)d->totals[0] > d->capV || (long long)d->totals[1] > d->capT) continue;
         if (item - __ldg(&first[q]) >= (uint32_t)d->gen_ngroups * (uint32_t)d->gen_nkc) continue;  // past its items
         const Grid g = d->g;
+        unsigned long long* out = s_out[threadIdx.x >> 5];
+        __syncwarp();  // the item before has written its last triangle
+        if ((threadIdx.x & 31) == 0) {
+            out[0] = reinterpret_cast<unsigned long long>(d->points);
+            out[1] = reinterpret_cast<unsigned long long>(d->tris);
+        }
+        __syncwarp();
         RowStarts rs;
         rs.starts = d->starts;
         rs.R = g.R;
@@ -495,7 +521,7 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells_batch(
         rs.add[0] = rs.add[1] = rs.add[2] = rs.add[3] = 0;
         gen_cells_item<IndexT, kGenFE, 0>(item - __ldg(&first[q]), s_raw, ws, tabs, d->bits, g, gen_lane(g, 32 / g.W, false),
                                        32 / g.W, GenCols{0, 1, d->gen_KC}, d->gen_ngroups, g.kr, g.ke, g.kr, 0ull, 0ull, d->row4, rs,
-                                       d->points, static_cast<IndexT*>(d->tris), nullptr, reverse);
+                                       GenOutShared<IndexT>{out}, nullptr, reverse);
     }
 }
 

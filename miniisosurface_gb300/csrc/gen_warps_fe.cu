@@ -117,7 +117,7 @@ void launch_gen_batch(int index_bytes, const BatchReq* reqs, const int* list, co
                       unsigned nitems, const CaseTables* cases, unsigned* work, int ws_bytes, int reverse, int nsm,
                       cudaStream_t s)
 {
-    const int warps = gen_cells_warps(ws_bytes, sizeof(GenCellTables<kGenFE>));
+    const int warps = std::min(kGenBatchWarps, gen_cells_warps(ws_bytes, sizeof(GenCellTables<kGenFE>) + 16 * kGenBatchWarps));
     const long long blocks = std::min(((long long)nitems + warps - 1) / warps, 2ll * nsm);
     if (blocks < 1) return;
     const size_t smem = (size_t)warps * ws_bytes;
