@@ -183,49 +183,77 @@ __global__ void k_block_tris(const uint32_t* __restrict__ bits, Grid g, BlockDim
 }
 
 // ---- the network -----------------------------------------------------------
-// A CTA of 512 threads takes tiles of 64 samples.  Everything that is summed over
+// A CTA of 256 threads takes tiles of 64 samples.  Everything that is summed over
 // is the slow index in shared memory (x, h1, d2, d1 by input or unit, 64 samples
 // side by side; the weights by input, 64 units side by side), so that a thread
-// makes a 4 x 2 part of a product from a 16-byte and an 8-byte load per term: warp
-// w the samples 4 w on, lane l the units 2 l and 2 l + 1.  The weight gradients are
-// sums over the samples: a thread makes those of units w + 16 a by l + 32 b from
-// 16-byte loads of four samples, in registers over all tiles of the CTA; eight
-// CTAs of a cluster then add theirs up through distributed shared memory, so that
-// a gradient gets one global addition per cluster instead of one per CTA (1.6
-// million on 6,401 addresses for 16,384 samples).  Sums are fused multiply-adds.
-// What bounds it, for 16,384 samples (256 tiles; 38 us, 106 with a row of 16 units
-// per thread and every CTA's own additions): issue in the tiles (24 us, 57 thousand
-// instructions each), latency in the rest (the weights' way in, five barriers a
-// tile, the cluster's end: 13 us).  Half the threads with 4 x 4 parts: 41 us.
+// makes a 4 x 4 part of a product from two 16-byte loads per term; a warp's lanes
+// cover 32 samples by 16 units.  The weight gradients are sums over the samples: a
+// thread makes those of 4 (of the first layer 3) units by 4 of the next layer from
+// 16-byte loads of four samples, two samples per instruction, in registers over
+// all tiles of the CTA; eight CTAs of a cluster then add theirs up through
+// distributed shared memory, so that a gradient gets one global addition per
+// cluster instead of one per CTA (1.6 million on 6,401 addresses for 16,384
+// samples).  Sums are fused multiply-adds.
+// What bounds it, for 16,384 samples (256 tiles; 34 us, 38 with 512 threads of 4 x
+// 2, 106 with a row of 16 units per thread and every CTA's own additions): the
+// bytes that shared memory returns to registers (a broadcast counts like any other
+// load; 0.5 floats per multiply-add, 0.75 with 4 x 2), then the latency of the
+// weights' way in, five barriers a tile and the cluster's end.
 constexpr int kTile = 64, kRow = kTile + 4;  // samples of a tile; of a row in shared memory (16-byte aligned)
 constexpr int kMlpCluster = 8;
-constexpr int kUnitRow = kHid + 2;
-constexpr int kMlpThreads = 512;
+constexpr int kUnitRow = kHid + 4;
+constexpr int kMlpThreads = 256;
 
 struct __align__(16) MlpSmem {
     float w1[kIn * kHid], w2[kHid * kHid], b1[kHid], b2[kHid], w3[kHid], b3[4];
     float x[kIn * kRow], h1[kHid * kRow];
-    float y[kTile];
+    float yp[4 * kTile];                    // the outputs' parts, by group of 16 units
 };
 
 struct __align__(16) MlpGradSmem {
     MlpSmem f;
-    float w2t[kHid * kUnitRow];             // w2 by unit of the second layer, rows two floats apart in the banks
+    float w2t[kHid * kUnitRow];             // w2 by unit of the second layer, rows four floats apart in the banks
     float d2[kHid * kRow], d1[kHid * kRow];
-    float dy[kTile], w3p[16 * kHid];        // each warp's part of dW3
+    float dy[kTile], w3p[2 * kHid];         // the two sample halves' parts of dW3
 };
 static_assert(sizeof(float) * kParams <= sizeof(float) * 2 * kHid * kRow, "a CTA's gradients fit over d2 and d1");
 
-__device__ __forceinline__ void load_params(MlpSmem& s, const float* __restrict__ p)
+// The parameters into shared memory, w2t (if any) the second layer's weights by its unit. Unrolled, so that a thread's
+// loads are on their way together.
+__device__ __forceinline__ void load_params(MlpSmem& s, const float* __restrict__ p, float* w2t = nullptr)
 {
-    for (int i = threadIdx.x; i < kIn * kHid; i += blockDim.x) s.w1[i] = p[i];
-    for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) s.w2[i] = p[kOffW2 + i];
-    for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
-        s.b1[i] = p[kOffB1 + i];
-        s.b2[i] = p[kOffB2 + i];
-        s.w3[i] = p[kOffW3 + i];
+    const int t = threadIdx.x;
+    static_assert(kHid * kHid % kMlpThreads == 0, "");
+#pragma unroll
+    for (int q = 0; q < kHid * kHid; q += kMlpThreads) {
+        const int i = q + t;
+        const float w = __ldg(p + kOffW2 + i);
+        s.w2[i] = w;
+        if (w2t) w2t[(i % kHid) * kUnitRow + i / kHid] = w;
     }
-    if (threadIdx.x == 0) s.b3[0] = p[kOffB3];
+#pragma unroll
+    for (int q = 0; q < kIn * kHid; q += kMlpThreads)
+        if (q + t < kIn * kHid) s.w1[q + t] = __ldg(p + q + t);
+    if (t < kHid) {
+        s.b1[t] = __ldg(p + kOffB1 + t);
+        s.b2[t] = __ldg(p + kOffB2 + t);
+        s.w3[t] = __ldg(p + kOffW3 + t);
+    }
+    if (t == 0) s.b3[0] = __ldg(p + kOffB3);
+}
+
+// A thread's 4 x 4 part of a tile: warp w the samples 32 (w & 1) on and units 16 (w >> 1) on, lane l of them 4 (l >> 2)
+// and 4 (l & 3) on.
+__device__ __forceinline__ int part_row() { return 32 * ((threadIdx.x >> 5) & 1) + 4 * ((threadIdx.x & 31) >> 2); }
+__device__ __forceinline__ int part_col() { return 16 * (threadIdx.x >> 6) + 4 * (threadIdx.x & 3); }
+
+// Output of the tile's sample r, after forward_tile.
+__device__ __forceinline__ float tile_y(const MlpSmem& s, int r)
+{
+    float y = s.b3[0];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) y += s.yp[q * kTile + r];
+    return y;
 }
 
 // Input c of a block's statistics st for the isovalue iso.
@@ -240,8 +268,10 @@ __device__ __forceinline__ float mlp_input(const float* __restrict__ st, float i
 __device__ __forceinline__ void load_tile(MlpSmem& s, const float* __restrict__ stats, const float* __restrict__ iso,
                                           long long base, long long n)
 {
-    for (int i = threadIdx.x; i < kTile * kIn; i += blockDim.x) {
-        const int r = i / kIn, c = i % kIn;
+#pragma unroll
+    for (int i0 = 0; i0 < kTile * kIn; i0 += kMlpThreads) {
+        const int i = i0 + threadIdx.x, r = i / kIn, c = i % kIn;
+        if (kTile * kIn % kMlpThreads != 0 && i >= kTile * kIn) break;
         const long long q = base + r;
         s.x[c * kRow + r] = q < n ? mlp_input(stats + q * kIn, iso[q], c) : 0.f;
     }
@@ -250,39 +280,49 @@ __device__ __forceinline__ void load_tile(MlpSmem& s, const float* __restrict__ 
 // out[b][a] = the product's value for sample r0 + a and unit c0 + b: bias + sum over K of in[k][sample] w[k][unit].
 template <int K, int WROW = kHid>
 __device__ __forceinline__ void mlp_product(const float* in, const float* w, const float* bias, int r0, int c0,
-                                            float (&out)[2][4])
+                                            float (&out)[4][4])
 {
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int a = 0; a < 4; ++a) out[b][a] = bias ? bias[c0 + b] : 0.f;
 #pragma unroll 8
     for (int k = 0; k < K; ++k) {
         const float4 xv = *reinterpret_cast<const float4*>(in + k * kRow + r0);
-        const float2 wv = *reinterpret_cast<const float2*>(w + k * WROW + c0);
-        const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[2] = {wv.x, wv.y};
+        const float4 wv = *reinterpret_cast<const float4*>(w + k * WROW + c0);
+        const float xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
+        for (int b = 0; b < 4; ++b)
 #pragma unroll
             for (int a = 0; a < 4; ++a) out[b][a] = __fmaf_rn(xs[a], ws[b], out[b][a]);
     }
 }
 
-__device__ __forceinline__ void store_units(float* o, int r0, int c0, const float (&v)[2][4])
+// Two fused multiply-adds at once, and the sum of a pair.
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v)
+{
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+
+__device__ __forceinline__ void store_units(float* o, int r0, int c0, const float (&v)[4][4])
 {
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < 4; ++b)
         *reinterpret_cast<float4*>(o + (c0 + b) * kRow + r0) = make_float4(v[b][0], v[b][1], v[b][2], v[b][3]);
 }
 
-// h1 (in shared memory), h2 (the thread's 4 x 2 part) and the output y of the tile.
-__device__ __forceinline__ void forward_tile(MlpSmem& s, float (&h2)[2][4])
+// h1 (in shared memory), h2 (the thread's 4 x 4 part) and the parts of the outputs of the tile.
+__device__ __forceinline__ void forward_tile(MlpSmem& s, float (&h2)[4][4])
 {
-    const int r0 = 4 * (threadIdx.x >> 5), c0 = 2 * (threadIdx.x & 31);
-    float h1[2][4];
+    const int r0 = part_row(), c0 = part_col();
+    float h1[4][4];
     mlp_product<kIn>(s.x, s.w1, s.b1, r0, c0, h1);
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int a = 0; a < 4; ++a) h1[b][a] = fmaxf(h1[b][a], 0.f);
     store_units(s.h1, r0, c0, h1);
@@ -290,7 +330,7 @@ __device__ __forceinline__ void forward_tile(MlpSmem& s, float (&h2)[2][4])
     mlp_product<kHid>(s.h1, s.w2, s.b2, r0, c0, h2);
     float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             h2[b][a] = fmaxf(h2[b][a], 0.f);
@@ -299,9 +339,10 @@ __device__ __forceinline__ void forward_tile(MlpSmem& s, float (&h2)[2][4])
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) part[a] += __shfl_xor_sync(0xffffffffu, part[a], d);
-        if ((threadIdx.x & 31) == 0) s.y[r0 + a] = part[a] + s.b3[0];
+        for (int d = 1; d < 4; d <<= 1) part[a] += __shfl_xor_sync(0xffffffffu, part[a], d);
     }
+    if ((threadIdx.x & 3) == 0)
+        *reinterpret_cast<float4*>(s.yp + (c0 / 16) * kTile + r0) = make_float4(part[0], part[1], part[2], part[3]);
     __syncthreads();
 }
 
@@ -314,9 +355,9 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_forward(const float* __rest
     for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
         load_tile(s, stats, iso, base, n);
         __syncthreads();
-        float h2[2][4];
+        float h2[4][4];
         forward_tile(s, h2);
-        if (threadIdx.x < kTile && base + threadIdx.x < n) y[base + threadIdx.x] = s.y[threadIdx.x];
+        if (threadIdx.x < kTile && base + threadIdx.x < n) y[base + threadIdx.x] = tile_y(s, threadIdx.x);
     }
 }
 
@@ -357,18 +398,20 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_predict(const float* __rest
             s_set[threadIdx.x] = set;
         }
         if (!__syncthreads_or(threadIdx.x < kTile && s_set[threadIdx.x] >= 0)) continue;  // no active block
-        for (int i = threadIdx.x; i < kTile * kIn; i += blockDim.x) {
-            const int r = i / kIn, c = i % kIn;
+#pragma unroll
+        for (int i0 = 0; i0 < kTile * kIn; i0 += kMlpThreads) {
+            const int i = i0 + threadIdx.x, r = i / kIn, c = i % kIn;
+            if (kTile * kIn % kMlpThreads != 0 && i >= kTile * kIn) break;
             const int set = s_set[r];
             s.x[c * kRow + r] =
                 set >= 0 ? mlp_input(sets.stats[set] + (base + r - sets.start[set]) * kIn, sets.iso[set], c) : 0.f;
         }
         __syncthreads();
-        float h2[2][4];
+        float h2[4][4];
         forward_tile(s, h2);
         if (threadIdx.x < 32) {  // the sets of a tile are neighbours
             const int lane = threadIdx.x, a = s_set[lane], b = s_set[lane + 32];
-            const float ya = a >= 0 ? fmaxf(s.y[lane], 0.f) : 0.f, yb = b >= 0 ? fmaxf(s.y[lane + 32], 0.f) : 0.f;
+            const float ya = a >= 0 ? fmaxf(tile_y(s, lane), 0.f) : 0.f, yb = b >= 0 ? fmaxf(tile_y(s, lane + 32), 0.f) : 0.f;
             const int none = sets.n;
             int q = __reduce_min_sync(0xffffffffu, min(a >= 0 ? a : none, b >= 0 ? b : none));
             while (q < none) {
@@ -392,22 +435,24 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     MlpGradSmem& s = *reinterpret_cast<MlpGradSmem*>(s_raw);
-    const int t = threadIdx.x, ty = t >> 5, tx = t & 31, r0 = 4 * ty, c0 = 2 * tx;
-    load_params(s.f, params);
-    for (int i = t; i < kHid * kHid; i += kMlpThreads) s.w2t[(i % kHid) * kUnitRow + i / kHid] = params[kOffW2 + i];
-    float gw2[4][2] = {}, gw1[3][2] = {}, gw3[2] = {};
+    const int t = threadIdx.x, r0 = part_row(), c0 = part_col();
+    // weight gradients: units i = gi + 16 a of one layer by l = gl + 32 b of the next
+    const int gi = 4 * ((t >> 5) & 3) + ((t & 31) >> 3), gl = 8 * (t >> 7) + (t & 7);
+    load_params(s.f, params, s.w2t);
+    unsigned long long gw2[4][4] = {}, gw1[3][4] = {};  // two sums each, of the even and of the odd samples
+    float gw3[4] = {};
     float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, lsum = 0.f;
     const float inv_n = 1.f / (float)n;
     for (long long base = (long long)blockIdx.x * kTile; base < n; base += (long long)gridDim.x * kTile) {
         load_tile(s.f, stats, iso, base, n);
         __syncthreads();
-        float h2[2][4];
+        float h2[4][4];
         forward_tile(s.f, h2);
         if (t < kTile) {
             const long long q = base + t;
             float dy = 0.f;
             if (q < n) {
-                const float e = s.f.y[t] - target[q];
+                const float e = tile_y(s.f, t) - target[q];
                 lsum = __fmaf_rn(e, e, lsum);
                 dy = 2.f * e * inv_n;
             }
@@ -416,12 +461,12 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
         }
         __syncthreads();
         // d2 = dy * w3 where h2 > 0; dW3 += h2 dy
-        float d[2][4];
+        float d[4][4];
         {
             const float4 dv = *reinterpret_cast<const float4*>(s.dy + r0);
             const float dys[4] = {dv.x, dv.y, dv.z, dv.w};
 #pragma unroll
-            for (int b = 0; b < 2; ++b)
+            for (int b = 0; b < 4; ++b)
 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
                     d[b][a] = h2[b][a] > 0.f ? dys[a] * s.f.w3[c0 + b] : 0.f;
@@ -433,7 +478,7 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
         // d1[sample][i] = sum_u d2[sample][u] w2[i][u] where h1 > 0
         mlp_product<kHid, kUnitRow>(s.d2, s.w2t, nullptr, r0, c0, d);
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < 4; ++b) {
             const float4 hv = *reinterpret_cast<const float4*>(s.f.h1 + (c0 + b) * kRow + r0);
             d[b][0] = hv.x > 0.f ? d[b][0] : 0.f;
             d[b][1] = hv.y > 0.f ? d[b][1] : 0.f;
@@ -443,31 +488,33 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
         store_units(s.d1, r0, c0, d);
         __syncthreads();
         // the tile's weight gradients, four samples at a time
-#pragma unroll 2
+#pragma unroll 1
         for (int r = 0; r < kTile; r += 4) {
-            float4 hv[4], dv[2];
+            ulonglong2 hv[4], dv[4];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) hv[a] = *reinterpret_cast<const float4*>(s.f.h1 + (ty + 16 * a) * kRow + r);
+            for (int a = 0; a < 4; ++a) hv[a] = *reinterpret_cast<const ulonglong2*>(s.f.h1 + (gi + 16 * a) * kRow + r);
 #pragma unroll
-            for (int b = 0; b < 2; ++b) dv[b] = *reinterpret_cast<const float4*>(s.d2 + (tx + 32 * b) * kRow + r);
+            for (int b = 0; b < 4; ++b) dv[b] = *reinterpret_cast<const ulonglong2*>(s.d2 + (gl + 16 * b) * kRow + r);
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    gw2[a][b] = __fmaf_rn(hv[a].x, dv[b].x, __fmaf_rn(hv[a].y, dv[b].y, __fmaf_rn(hv[a].z, dv[b].z,
-                                          __fmaf_rn(hv[a].w, dv[b].w, gw2[a][b]))));
+                for (int b = 0; b < 4; ++b) {
+                    fma_pair(gw2[a][b], hv[a].x, dv[b].x);
+                    fma_pair(gw2[a][b], hv[a].y, dv[b].y);
+                }
 #pragma unroll
             for (int a = 0; a < 3; ++a)
-                hv[a] = ty + 16 * a < kIn ? *reinterpret_cast<const float4*>(s.f.x + (ty + 16 * a) * kRow + r)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+                hv[a] = gi + 16 * a < kIn ? *reinterpret_cast<const ulonglong2*>(s.f.x + (gi + 16 * a) * kRow + r)
+                                          : make_ulonglong2(0ull, 0ull);
 #pragma unroll
-            for (int b = 0; b < 2; ++b) dv[b] = *reinterpret_cast<const float4*>(s.d1 + (tx + 32 * b) * kRow + r);
+            for (int b = 0; b < 4; ++b) dv[b] = *reinterpret_cast<const ulonglong2*>(s.d1 + (gl + 16 * b) * kRow + r);
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    gw1[a][b] = __fmaf_rn(hv[a].x, dv[b].x, __fmaf_rn(hv[a].y, dv[b].y, __fmaf_rn(hv[a].z, dv[b].z,
-                                          __fmaf_rn(hv[a].w, dv[b].w, gw1[a][b]))));
+                for (int b = 0; b < 4; ++b) {
+                    fma_pair(gw1[a][b], hv[a].x, dv[b].x);
+                    fma_pair(gw1[a][b], hv[a].y, dv[b].y);
+                }
         }
         if (t < 2 * kHid) {  // db1, db2: one unit's samples per thread
             const float* row = t < kHid ? s.d1 + t * kRow : s.d2 + (t - kHid) * kRow;
@@ -486,16 +533,20 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b) own[kOffW2 + (ty + 16 * a) * kHid + tx + 32 * b] = gw2[a][b];
+        for (int b = 0; b < 4; ++b) own[kOffW2 + (gi + 16 * a) * kHid + gl + 16 * b] = pair_sum(gw2[a][b]);
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-            if (ty + 16 * a < kIn) own[(ty + 16 * a) * kHid + tx + 32 * b] = gw1[a][b];
+        for (int b = 0; b < 4; ++b)
+            if (gi + 16 * a < kIn) own[(gi + 16 * a) * kHid + gl + 16 * b] = pair_sum(gw1[a][b]);
     if (t < kHid) own[kOffB1 + t] = gb1;
     else if (t < 2 * kHid) own[kOffB2 + t - kHid] = gb2;
 #pragma unroll
-    for (int b = 0; b < 2; ++b) s.w3p[ty * kHid + c0 + b] = gw3[b];  // dW3: the warps' parts
+    for (int b = 0; b < 4; ++b) {  // dW3: a warp's samples, then the halves
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) gw3[b] += __shfl_xor_sync(0xffffffffu, gw3[b], d);
+        if ((t & 31) < 4) s.w3p[((t >> 5) & 1) * kHid + c0 + b] = gw3[b];
+    }
     if (t < kTile) {  // db3 and the loss: two warps
         for (int d = 16; d > 0; d >>= 1) {
             gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
@@ -507,11 +558,7 @@ __global__ void __cluster_dims__(kMlpCluster, 1, 1) __launch_bounds__(kMlpThread
         }
     }
     __syncthreads();
-    if (t < kHid) {
-        float v = 0.f;
-        for (int w = 0; w < 16; ++w) v += s.w3p[w * kHid + t];
-        own[kOffW3 + t] = v;
-    }
+    if (t < kHid) own[kOffW3 + t] = s.w3p[t] + s.w3p[kHid + t];
     if (t == kHid) {
         own[kOffB3] = s.dy[0] + s.dy[1];
         atomicAdd(loss, (s.dy[2] + s.dy[3]) * inv_n);
