@@ -44,12 +44,12 @@ void replan(iso_ctx* ctx, std::vector<BatchItem>& items, const std::vector<int>&
 // Fused requests.  Flying Edges requests whose rows fit the multi-row kernels
 // (up to 16 words, the volume at a 16-byte boundary) run together, one launch
 // per pass and kernel variant (batch_kernels.cuh): the count blocks of every
-// request of a count variant, the two scan phases of all of them, the vertex
-// prefix, the generate items of every request of a generate variant (rows
-// per warp, index width), and one vertex pass over all their slots.  Each
-// request has its own scratch, so nothing is shared between requests but the
-// launches.  The descriptors and launch lists are written into pinned host
-// memory before every run and copied in by the first node.
+// request of a count variant (rows that are a multiple of 16 bytes, and
+// others), the two scan phases of all of them, the vertex prefix, the generate
+// items of every request of an index width, and one vertex pass over all their
+// slots.  Each request has its own scratch, so nothing is shared between
+// requests but the launches.  The descriptors and launch lists are written into
+// pinned host memory before every run and copied in by the first node.
 // ---------------------------------------------------------------------------
 struct FusedGroup {
     bool aligned = false;      // count: rows a multiple of 4 points

@@ -776,8 +776,6 @@ CountPlan count_plan(const Grid& g, int nsm)
     CountPlan p;
     p.J = kCountRows;
     p.nyb = (g.ny + p.J - 1) / p.J;
-    p.vec_u = 1;
-    while (p.vec_u * 128 < g.nx) p.vec_u <<= 1;  // float4 per lane for one row
     // ~8 CTAs per SM in total, at least 8 planes per column
     const int nzw = g.ke - g.kr;  // planes of the window
     const long long target = (long long)nsm * 8;

@@ -23,7 +23,6 @@
 
 namespace iso {
 
-constexpr int kTileRows = 256;     // grid rows per count/scan tile
 constexpr int kThreads = 256;      // threads per CTA of the row kernels
 
 struct Grid {
@@ -90,22 +89,6 @@ template <int G>
 __device__ __forceinline__ uint32_t group_bcast(uint32_t v, int src, unsigned mask)
 {
     return __shfl_sync(mask, v, src, G);
-}
-
-template <int G>
-__device__ __forceinline__ uint32_t group_min(uint32_t v, unsigned mask)
-{
-#pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) v = min(v, __shfl_xor_sync(mask, v, d, G));
-    return v;
-}
-
-template <int G>
-__device__ __forceinline__ uint32_t group_max(uint32_t v, unsigned mask)
-{
-#pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(mask, v, d, G));
-    return v;
 }
 
 // Value of the volume at grid point (i, j, k).
@@ -305,80 +288,6 @@ struct RowColWalk {
     }
 };
 
-// Bit mask "value >= iso" of rows [0, nrows) of nx values each (row stride
-// nx) into dst[row * W + w].  All threads of the CTA take part; SHARED
-// selects a shared-memory source (plain loads) or a global one (__ldg).
-template <bool VEC4, bool SHARED>
-__device__ __forceinline__ void classify_block(const float* __restrict__ src, int nx, int W, int nrows, float iso,
-                                               uint32_t* __restrict__ dst)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (VEC4) {
-        const int nq = nx >> 2, nq8 = (nq + 7) & ~7;
-        constexpr int U = 4;
-        RowColWalk it(tid, kThreads, nq8);
-        const int total = nrows * nq8;
-        for (int f0 = 0; f0 < total; f0 += U * kThreads) {
-            float4 v[U];
-            RowColWalk at = it;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool ok = at.row < nrows && at.col < nq;
-                const float4* p = reinterpret_cast<const float4*>(src + (size_t)at.row * nx) + at.col;
-                v[u] = ok ? (SHARED ? *p : __ldg(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                at.advance();
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool ok = it.row < nrows && it.col < nq;
-                const uint32_t nib = ok ? ((uint32_t)(v[u].x >= iso) | ((uint32_t)(v[u].y >= iso) << 1) |
-                                           ((uint32_t)(v[u].z >= iso) << 2) | ((uint32_t)(v[u].w >= iso) << 3))
-                                        : 0u;
-                uint32_t word = nib << (4 * (lane & 7));
-                word |= __shfl_xor_sync(0xffffffffu, word, 1);
-                word |= __shfl_xor_sync(0xffffffffu, word, 2);
-                word |= __shfl_xor_sync(0xffffffffu, word, 4);
-                if ((lane & 7) == 0 && ok) dst[it.row * W + (it.col >> 3)] = word;
-                it.advance();
-            }
-        }
-    } else {
-        constexpr int U = 4, NW = kThreads / 32;
-        RowColWalk it(warp, NW, W);
-        const int total = nrows * W;
-        for (int f0 = 0; f0 < total; f0 += U * NW) {
-            float v[U];
-            RowColWalk at = it;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int i = 32 * at.col + lane;
-                const bool ok = at.row < nrows && i < nx;
-                const float* p = src + (size_t)at.row * nx + i;
-                v[u] = ok ? (SHARED ? *p : __ldg(p)) : 0.f;
-                at.advance();
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int i = 32 * it.col + lane;
-                const bool ok = it.row < nrows && i < nx;
-                const uint32_t word = __ballot_sync(0xffffffffu, ok && v[u] >= iso);
-                if (lane == 0 && it.row < nrows) dst[it.row * W + it.col] = word;
-                it.advance();
-            }
-        }
-    }
-}
-
-// q = x / d for 0 <= x < 2^22 using a float reciprocal inv = 1/d and one
-// correction step (no integer division in hot loops).
-__device__ __forceinline__ int fastdiv(int x, int d, float inv)
-{
-    int q = __float2int_rz((float)x * inv);
-    if (q * d > x) --q;
-    else if ((q + 1) * d <= x) ++q;
-    return q;
-}
-
 // Low grid point and axis of cube edge e of cell (0,0,0).
 __device__ __forceinline__ void cube_edge_geometry(int e, int& dx, int& dy, int& dz, int& axis)
 {
@@ -465,11 +374,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity)
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 #ifdef ISO_WAIT_STATS

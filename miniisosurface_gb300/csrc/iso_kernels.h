@@ -22,8 +22,8 @@ struct FeBuffers {
     uint32_t* mccnt = nullptr;             // R      MC vertices per cell row
     unsigned long long* starts = nullptr;  // 4*R    per row: first vertex, triangle, MC vertex (or y, z cuts)
     unsigned long long* part = nullptr;    // 4*nseg scan segment totals
-    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts
-    uint32_t* bits = nullptr;              // R*W    bit rows (row-wise kernels only)
+    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, -, work counter
+    uint32_t* bits = nullptr;              // R*W    bit rows
     uint32_t* fe2mc = nullptr;             // >= V   FE vertex index -> MC index
 };
 
@@ -32,7 +32,6 @@ struct FeBuffers {
 // the row scans.
 struct CountPlan {
     int J = 8, nyb = 1, KC = 1, nkc = 1;
-    int vec_u = 1;  // float4 loads per lane for one row (rows up to 64 words)
     int nseg = 1;
     int nsm = 0;      // SMs of the device the plan is for
     bool trims = false;  // write the row trims (only the pass-by-pass interface reads them)
