@@ -26,8 +26,8 @@
 //
 // What bounds it: instruction issue (77% of the slots on the 512^3 volume, with 117 M warp instructions; the kernels
 // it replaced, which recomputed eight masks and four scans per row and step, took 161 M).  Events around the pass, us,
-// Flying Edges, before / now: 512^3 167 / 128, 768^3 (with the vertices, which were in the same kernel) 1252 / 722,
-// 667 x 228 x 724 the same 363 / 208, 150 x 700 x 600 110 / 70, 301 x 217 x 190 36 / 28, 128^3 22 / 16.6, 64^3 17 / 13.3.
+// Flying Edges, before / now: 512^3 167 / 124, 768^3 (with the vertices, which were in the same kernel) 1252 / 715,
+// 667 x 228 x 724 the same 363 / 208, 150 x 700 x 600 110 / 68, 301 x 217 x 190 36 / 27, 128^3 22 / 16.5, 64^3 17 / 12.
 // Three rows per lane and one more instead of two and one: 145 us at 512^3 (fewer warps fit).  Vertex runs made dense like the cells
 // instead of a loop over each word's bits: 32 M instructions instead of 21 M.
 // Marching Cubes: a cell away from the first column, row and plane owns at most three vertices, read ready from a
@@ -42,7 +42,10 @@ namespace iso {
 
 constexpr int kGenSlots = 2;       // rows per lane
 constexpr int kGenExtra = 2;       // rows side by side up to which a kernel for them gives the row after the group a slot
-constexpr int kGenChunk = 64;      // cells whose triangles are listed together
+// Cells whose triangles are listed together: a step of the 512^3 volume has 85, so that most take one list and the
+// triangles' batches are full but for its last (64 cells: 126.3 us, 96: 123.7, 128: 123.8; 301 x 217 x 190 28.3 / 26.8 /
+// 26.8, 64^3 12.8 / 12.0 / 12.0). Marching Cubes: 64, so that their vertices fit their list (kGenOwned).
+__host__ __device__ inline constexpr int gen_chunk(int mode) { return mode == kGenFE ? 96 : 64; }
 constexpr int kGenMaxWarps = 16;   // warps per CTA, two CTAs per SM
 // ... of the batch kernel, which holds what others take from their parameters in registers: with 16 it spilled 29 of
 // them (64 uneven volumes, whole call 2030 us; 14: 1960, 12: 1970, 10: 2013)
@@ -60,10 +63,10 @@ __host__ __device__ inline int gen_word_entries(int rpw) { return kGenSlots * rp
 __host__ __device__ inline bool gen_owns(int mode) { return mode == kGenMC || mode == kGenMCT; }
 __host__ __device__ inline int gen_cells_scratch(int W, int rpw, int mode)
 {
-    const int list = mode == kGenMC ? 0 : 5 * kGenChunk * 2;
-    const int own = gen_owns(mode) ? 4 * kGenChunk + 2 * kGenOwned : 0;
+    const int list = mode == kGenMC ? 0 : 5 * gen_chunk(mode) * 2;
+    const int own = gen_owns(mode) ? 4 * gen_chunk(mode) + 2 * kGenOwned : 0;
     // + 48: the last row of a slot looks one entry past its word's rows
-    return (64 * W * gen_word_entries(rpw) + 48 + 4 * kGenChunk + list + own + 15) & ~15;
+    return (64 * W * gen_word_entries(rpw) + 48 + 4 * gen_chunk(mode) + list + own + 15) & ~15;
 }
 
 // The kernel's per-case tables in shared memory (CaseTables holds them ready).
@@ -184,6 +187,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
 {
     constexpr bool OWNS = GenCellTables<MODE>::OWNS, TRIS = GenCellTables<MODE>::TRIS;
     constexpr bool WIDE = MODE == kGenFE && sizeof(IndexT) == 8;  // ids past 32 bits; the map's ids are 32-bit
+    constexpr int kChunk = gen_chunk(MODE);
     constexpr int S = kGenSlots, NS = S + (gen_extra_slot(RPW) ? 1 : 0);
     static_assert(S == 2, "the active cells' counts of a lane's slots share a word");
     const int rpw = RPW > 0 ? RPW : rpw_;
@@ -193,9 +197,9 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
     unsigned char* tab = s_raw + ws;
     unsigned char* pair = tab + 48 * W * E;
     uint32_t* cell = reinterpret_cast<uint32_t*>(pair + 16 * W * E + 48);
-    uint16_t* list = reinterpret_cast<uint16_t*>(cell + kGenChunk);
-    uint32_t* place = reinterpret_cast<uint32_t*>(list + (TRIS ? 5 * kGenChunk : 0));
-    uint16_t* vlist = reinterpret_cast<uint16_t*>(place + kGenChunk);
+    uint16_t* list = reinterpret_cast<uint16_t*>(cell + kChunk);
+    uint32_t* place = reinterpret_cast<uint32_t*>(list + (TRIS ? 5 * kChunk : 0));
+    uint16_t* vlist = reinterpret_cast<uint16_t*>(place + kChunk);
 
     const int col = (int)(item / (uint32_t)ngroups);
     const int jw = G * (int)(item - (uint32_t)col * (uint32_t)ngroups);
@@ -319,8 +323,8 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
             const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
             const uint32_t tot0 = tot & 0xffffu, ctot = tot0 + (tot >> 16);
             // the owned vertices of a chunk fit their list: a cell owns at most 12 on the first plane and row, else 5
-            const uint32_t chunk = OWNS && (k == 0 || jw == 0) ? 32u : (uint32_t)kGenChunk;
-            static_assert(kGenOwned >= 12 * 32 && kGenOwned >= 5 * kGenChunk, "owned vertices of a chunk");
+            const uint32_t chunk = OWNS && (k == 0 || jw == 0) ? 32u : (uint32_t)kChunk;
+            static_assert(!OWNS || (kGenOwned >= 12 * 32 && kGenOwned >= 5 * kChunk), "owned vertices of a chunk");
             for (uint32_t c0 = 0; c0 < ctot; c0 += chunk) {
                 uint32_t ntri = 0, nown = 0;
 #pragma unroll 1
@@ -367,7 +371,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                         const uint32_t me = cb + (uint32_t)lane;
 #pragma unroll
                         for (uint32_t q = 0; q < 5; ++q)
-                            if (q < nt) l[q] = (uint16_t)(me | (q << 6));
+                            if (q < nt) l[q] = (uint16_t)(me | (q << 7));
                         ntri += __shfl_sync(0xffffffffu, it, 31);
                     }
                     if (OWNS) {
@@ -387,12 +391,12 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                             const uint64_t ord = tabs.order[cs];
                             for (int q = 0; q < iso_case_ntris(ord); ++q) {
                                 const int ed = iso_case_edge(ord, q);
-                                if ((own >> ed) & 1u) *o++ = (uint16_t)(me | ((uint32_t)ed << 6));
+                                if ((own >> ed) & 1u) *o++ = (uint16_t)(me | ((uint32_t)ed << 7));
                             }
                         } else {
-                            if (no > 0u) o[0] = (uint16_t)(me | ((ready >> 2) & 0x3c0u));
-                            if (no > 1u) o[1] = (uint16_t)(me | ((ready >> 6) & 0x3c0u));
-                            if (no > 2u) o[2] = (uint16_t)(me | ((ready >> 10) & 0x3c0u));
+                            if (no > 0u) o[0] = (uint16_t)(me | ((ready >> 1) & 0x780u));
+                            if (no > 1u) o[1] = (uint16_t)(me | ((ready >> 5) & 0x780u));
+                            if (no > 2u) o[2] = (uint16_t)(me | ((ready >> 9) & 0x780u));
                         }
                         nown += __shfl_sync(0xffffffffu, io, 31);
                     }
@@ -401,8 +405,8 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                 if (OWNS) {
                     for (uint32_t v = (uint32_t)lane; v < nown; v += 32) {
                         const uint32_t vr = vlist[v];
-                        const uint32_t cr = cell[vr & 63u], pl = place[vr & 63u];
-                        const int e12 = (int)(vr >> 6);
+                        const uint32_t cr = cell[vr & 127u], pl = place[vr & 127u];
+                        const int e12 = (int)(vr >> 7);
                         const unsigned long long mid = mcur + v;
                         int dx, dy, dz, axis;
                         cube_edge_geometry(e12, dx, dy, dz, axis);
@@ -422,8 +426,8 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                     IndexT* o = out.tris() + 3 * (tcur + (uint32_t)lane - tbase);
                     for (uint32_t t = (uint32_t)lane; t < ntri; t += 32, o += 96) {
                         const uint32_t c = list[t];
-                        const uint32_t rec = cell[c & 63u];
-                        const uint32_t corners = tabs.corner[(rec >> 18) + (c >> 6)];
+                        const uint32_t rec = cell[c & 127u];
+                        const uint32_t corners = tabs.corner[(rec >> 18) + (c >> 7)];
                         const uint32_t at = ws + (rec & 0x1fffu), sft = 32u - ((rec >> 13) & 31u);
                         uint32_t vid[3];
 #pragma unroll
