@@ -24,7 +24,7 @@
 // is the same byte for every grid (axis * 16 + row * 48 + plane * 8, bit 0 the
 // edge at point i + 1), and the other plane is bit 3 of the address.
 //
-// What bounds it: instruction issue (77% of the slots on the 512^3 volume, with 117 M warp instructions; the kernels
+// What bounds it: instruction issue (77% of the slots on the 512^3 volume, with 115 M warp instructions; the kernels
 // it replaced, which recomputed eight masks and four scans per row and step, took 161 M).  Events around the pass, us,
 // Flying Edges, before / now: 512^3 167 / 124, 768^3 (with the vertices, which were in the same kernel) 1252 / 715,
 // 667 x 228 x 724 the same 363 / 208, 150 x 700 x 600 110 / 68, 301 x 217 x 190 36 / 27, 128^3 22 / 16.5, 64^3 17 / 12.
