@@ -395,8 +395,8 @@ __device__ __forceinline__ void scan_publish(unsigned long long* __restrict__ to
         publish[0] = v;
         publish[1] = t;
         publish[2] = m;
-        publish[3] = totals[3];
-        totals[3] = 0;
+        publish[3] = totals[kStatusKept];
+        totals[kStatusKept] = 0;
     }
 }
 
@@ -817,7 +817,7 @@ CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned
 
 template <bool MC>
 static void count_launch(const CountPlan& p, const float* vol, const Grid& g, float iso, const CaseTables* cases,
-                         FeBuffers& b, cudaStream_t s)
+                         FeBuffers& b, unsigned long long* status, cudaStream_t s)
 {
     const unsigned blocks = (unsigned)(p.nyb * p.nkc);
     const bool base16 = (reinterpret_cast<uintptr_t>(vol) & 15) == 0;
@@ -833,7 +833,7 @@ static void count_launch(const CountPlan& p, const float* vol, const Grid& g, fl
                              : (aligned ? k_count_rows<MC, 1, true> : k_count_rows<MC, 1, false>);
         allow_smem(kern, smem);
         kern<<<nb, kCountThreads, smem, s>>>(vol, g, count_below(iso), r.KC, r.groups, r.items, r.stage, b.rowcnt,
-                                             trims, b.mccnt, b.bits, b.totals + 3);
+                                             trims, b.mccnt, b.bits, status);
         return;
     }
     if (g.W > 64) {
@@ -857,9 +857,9 @@ static void count_launch(const CountPlan& p, const float* vol, const Grid& g, fl
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
                   const CountPlan& p, FeBuffers& b, cudaStream_t s, bool zero_status)
 {
-    if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
-    if (mc) count_launch<true>(p, vol, g, iso, cases, b, s);
-    else count_launch<false>(p, vol, g, iso, cases, b, s);
+    unsigned long long* status = count_status(b, zero_status, s);
+    if (mc) count_launch<true>(p, vol, g, iso, cases, b, status, s);
+    else count_launch<false>(p, vol, g, iso, cases, b, status, s);
 }
 
 BatchCount batch_count(const Grid& g, int planes)

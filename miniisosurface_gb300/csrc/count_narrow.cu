@@ -161,7 +161,8 @@ bool narrow_fits(const Grid& g, const void* vol, int dtype)
 }
 
 template <bool MC, typename S>
-static void narrow_launch(const CountPlan& p, const S* vol, const Grid& g, int thr, FeBuffers& b, cudaStream_t s)
+static void narrow_launch(const CountPlan& p, const S* vol, const Grid& g, int thr, FeBuffers& b,
+                          unsigned long long* status, cudaStream_t s)
 {
     const bool aligned = g.nx * (int)sizeof(S) % 16 == 0;
     const CountRows r = count_rows_plan(g, p.nsm, (int)sizeof(S), aligned, false);
@@ -172,18 +173,18 @@ static void narrow_launch(const CountPlan& p, const S* vol, const Grid& g, int t
                          : (aligned ? k_count_narrow<MC, S, 1, true> : k_count_narrow<MC, S, 1, false>);
     allow_smem(kern, smem);
     kern<<<nb, kCountThreads, smem, s>>>(vol, g, thr, r.KC, r.groups, r.items, r.stage, b.rowcnt, b.mccnt, b.bits,
-                                         b.totals + 3);
+                                         status);
 }
 
 void launch_count_narrow(const void* vol, int dtype, const Grid& g, float iso, bool mc, const CountPlan& p, FeBuffers& b,
                          cudaStream_t s, bool zero_status)
 {
-    if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);  // device status
+    unsigned long long* status = count_status(b, zero_status, s);
     const int thr = narrow_threshold(iso);
 #define ISO_TYPE(T)                                                                   \
     {                                                                                 \
-        if (mc) narrow_launch<true, T>(p, static_cast<const T*>(vol), g, thr, b, s);  \
-        else narrow_launch<false, T>(p, static_cast<const T*>(vol), g, thr, b, s);    \
+        if (mc) narrow_launch<true, T>(p, static_cast<const T*>(vol), g, thr, b, status, s);  \
+        else narrow_launch<false, T>(p, static_cast<const T*>(vol), g, thr, b, status, s);    \
     }
     switch (dtype) {
         case ISO_INT8: ISO_TYPE(int8_t) break;

@@ -22,7 +22,7 @@ struct FeBuffers {
     uint32_t* mccnt = nullptr;             // R      MC vertices per cell row
     unsigned long long* starts = nullptr;  // 4*R    per row: first vertex, triangle, MC vertex (or y, z cuts)
     unsigned long long* part = nullptr;    // 4*nseg scan segment totals
-    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, -, work counter
+    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, kept status, work counter
     uint32_t* bits = nullptr;              // R*W    bit rows
     uint32_t* fe2mc = nullptr;             // >= V   FE vertex index -> MC index
 };
@@ -102,7 +102,14 @@ CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned
 GenPlan gen_plan(const Grid& g, int nsm);
 
 // passes 1-3
-// zero_status: the device status (totals[3]) is zeroed first; without it, it has to be zero (launch_scan's publish)
+// The device status of a count: totals[3], zeroed before it, or with zero_status off a word that the scan's publish
+// leaves at zero and nothing else writes (an extraction that does not publish leaves its own status behind).
+constexpr int kStatusKept = 6;
+inline unsigned long long* count_status(const FeBuffers& b, bool zero_status, cudaStream_t s)
+{
+    if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);
+    return b.totals + (zero_status ? 3 : kStatusKept);
+}
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
                   const CountPlan& p, FeBuffers& b, cudaStream_t s, bool zero_status = true);
 enum ScanMode { kScanFE = 0, kScanMC = 1, kScanDup = 2 };
