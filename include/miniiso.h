@@ -407,9 +407,10 @@ iso_status iso_vtk_write_mesh(const char* path, const iso_mesh* mesh);
 /* Writes a float32 volume as BINARY STRUCTURED_POINTS (big-endian). */
 iso_status iso_vtk_write_image(const char* path, const iso_grid* grid, const float* data);
 
-/* Brings the pages of n host ranges in, on all host threads, before a mesh is
- * copied into them; their contents stay. A hint: ISO_OK also where the system
- * cannot do it. */
+/* Brings the pages of n host ranges in before a mesh is copied into them; their
+ * contents stay. Helper threads end with the call; all callers together have three
+ * at most. A hint: ISO_OK also where the system cannot do
+ * it. */
 iso_status iso_populate_host(int64_t n, void* const* ptrs, const int64_t* bytes);
 
 /* ---- synthetic volumes of the benchmark configurations ---- */

@@ -183,7 +183,7 @@ def _host_mesh_buffers(nv, nt, index_bytes):
     m.points, m.normals, m.tris = pts.ctypes.data, nrm.ctypes.data, tri.ctypes.data
     m.index_bytes = index_bytes
     m.cap_points, m.cap_tris = nv, nt
-    if pts.nbytes + nrm.nbytes + tri.nbytes >= _POPULATE_BYTES:  # new memory: its pages brought in by all host threads
+    if pts.nbytes + nrm.nbytes + tri.nbytes >= _POPULATE_BYTES:  # new memory: its pages brought in by several host threads
         load().iso_populate_host(3, (C.c_void_p * 3)(m.points, m.normals, m.tris),
                                  (C.c_int64 * 3)(pts.nbytes, nrm.nbytes, tri.nbytes))
     return m, pts, nrm, tri
