@@ -921,6 +921,7 @@ iso_status iso_extract_device_typed(iso_ctx* ctx, iso_algorithm algo, const void
                                     const iso_grid* grid, float isoval, iso_mesh* out, void* stream)
 {
     if (!ctx || !grid || iso::dtype_bytes(dtype) == 0) return ISO_ERR_INVALID_ARG;
+    if (!valid_algo(algo)) return ISO_ERR_INVALID_ARG;
     if (dtype == ISO_FLOAT32) return iso_extract_device(ctx, algo, static_cast<const float*>(volume), grid, isoval,
                                                         out, stream);
     Grid g;
