@@ -573,6 +573,14 @@ iso_status iso_ctx_create(int device, iso_ctx** out)
             st = cuda_fail(ctx, e, "cudaMallocHost");
             break;
         }
+        // its own allocation, zeroed here: the scratch may grow within a capture, where a memset would not run
+        const unsigned long long zero = 0;
+        if ((e = cudaMalloc(&ctx->d_status, sizeof zero)) != cudaSuccess ||
+            (e = cudaMemcpy(ctx->d_status, &zero, sizeof zero, cudaMemcpyHostToDevice)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) {
+            st = cuda_fail(ctx, e, "the status word");
+            break;
+        }
     } while (0);
     if (st != ISO_OK) {
         iso_ctx_destroy(ctx);
@@ -588,6 +596,7 @@ iso_status iso_ctx_destroy(iso_ctx* ctx)
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
     cudaFree(ctx->d_cases);
+    cudaFree(ctx->d_status);
     cudaFree(ctx->scratch);
     cudaFree(ctx->fe2mc);
     cudaFree(ctx->d_volume);

@@ -35,6 +35,7 @@ struct iso_ctx {
     long long d_cap_points = 0, d_cap_tris = 0;
     int d_index_bytes = 0;
     unsigned long long* h_totals = nullptr;  // pinned, 4 entries
+    unsigned long long* d_status = nullptr;  // device status of the publishing calls, one word, zero between them
     unsigned long long* h_slab = nullptr;    // pinned and mapped, 2 x 9 entries (slab counts)
     unsigned long long* h_slab_dev = nullptr;  // its device address (written by k_slab_readback)
     void* scratch_b = nullptr;               // second scratch set (streamed path: the next slab's counts)
@@ -199,7 +200,7 @@ inline void carve(void* base, const Grid& g, const iso::CountPlan& cp, FeBuffers
 {
     const size_t R = (size_t)g.R;
     char* p = static_cast<char*>(base);
-    b.totals = reinterpret_cast<unsigned long long*>(p); p += align256(8 * 8);  // at one place whatever the grid
+    b.totals = reinterpret_cast<unsigned long long*>(p); p += align256(8 * 8);
     b.rowcnt = reinterpret_cast<uint4*>(p); p += align256(R * 16);
     b.row4 = reinterpret_cast<uint4*>(p); p += align256(R * 16);
     b.trims = reinterpret_cast<uint2*>(p); p += align256(R * 8);
@@ -222,9 +223,9 @@ inline iso_status ensure_scratch(iso_ctx* ctx, const Grid& g, const iso::CountPl
         const size_t alloc = need + need / 4;
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch, alloc));
         ctx->scratch_bytes = alloc;
-        ISO_CUDA(ctx, cudaMemsetAsync(ctx->scratch, 0, 8 * sizeof(unsigned long long), s));  // the device status
     }
     carve(ctx->scratch, g, cp, b);
+    b.kept = ctx->d_status;
     b.fe2mc = ctx->fe2mc;
     return ISO_OK;
 }
@@ -257,9 +258,9 @@ inline iso_status ensure_scratch_b(iso_ctx* ctx, const Grid& g, const iso::Count
         const size_t alloc = need + need / 4;
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch_b, alloc));
         ctx->scratch_b_bytes = alloc;
-        ISO_CUDA(ctx, cudaMemsetAsync(ctx->scratch_b, 0, 8 * sizeof(unsigned long long), s));
     }
     carve(ctx->scratch_b, g, cp, b);
+    b.kept = ctx->d_status;
     b.fe2mc = ctx->fe2mc;
     return ISO_OK;
 }
@@ -343,7 +344,7 @@ inline Plans make_plans(const iso_ctx* ctx, const Grid& g, int nsm = 0)
 }
 
 // Passes 1-3: counts, scan, row starts.  publish: the counts and the device status go there without a copy (pinned
-// host memory); the status is then the context's scratch's own, zero from call to call, and needs no memset.
+// host memory); the status is then the context's own word, zero from call to call, and needs no memset.
 inline void enqueue_count(iso_ctx* ctx, iso_algorithm algo, const float* vol, const Grid& g, float iso, const Plans& pl,
                    FeBuffers& b, cudaStream_t s, PassMarks& pm, unsigned long long* publish = nullptr)
 {

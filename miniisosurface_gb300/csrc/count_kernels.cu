@@ -388,15 +388,16 @@ __global__ void __launch_bounds__(kThreads) k_scan_partial(const uint4* __restri
 // to the host (launch_scan).
 __device__ __forceinline__ void scan_publish(unsigned long long* __restrict__ totals, unsigned long long v,
                                              unsigned long long t, unsigned long long m,
-                                             unsigned long long* __restrict__ publish)
+                                             unsigned long long* __restrict__ publish,
+                                             unsigned long long* __restrict__ kept)
 {
     totals[7] = 0;
     if (publish) {
         publish[0] = v;
         publish[1] = t;
         publish[2] = m;
-        publish[3] = totals[kStatusKept];
-        totals[kStatusKept] = 0;
+        publish[3] = *kept;
+        *kept = 0;
     }
 }
 
@@ -415,7 +416,8 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
                                                  const unsigned long long* __restrict__ part, int nseg,
                                                  unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
                                                  unsigned long long* __restrict__ totals,
-                                                 unsigned long long* __restrict__ publish, int blk)
+                                                 unsigned long long* __restrict__ publish,
+                                                 unsigned long long* __restrict__ kept, int blk)
 {
     constexpr int NC = ScanComps<SM>::n;
     __shared__ unsigned long long s_w[NC][kThreads / 32];
@@ -463,7 +465,7 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
             totals[4] = s_tot[0];
             totals[5] = e2;
         }
-        scan_publish(totals, V, s_tot[1], m, publish);
+        scan_publish(totals, V, s_tot[1], m, publish, kept);
     }
 #pragma unroll
     for (int a = 0; a < NC; ++a) {
@@ -513,11 +515,12 @@ __global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* __restrict
                                                          unsigned long long* __restrict__ starts,
                                                          uint4* __restrict__ row4,
                                                          unsigned long long* __restrict__ totals,
-                                                         unsigned long long* __restrict__ publish)
+                                                         unsigned long long* __restrict__ publish,
+                                                         unsigned long long* __restrict__ kept)
 {
     wait_for_previous();
     next_may_start();
-    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, row4, totals, publish, (int)blockIdx.x);
+    scan_final_block<SM>(rowcnt, mccnt, R, part, nseg, starts, row4, totals, publish, kept, (int)blockIdx.x);
 }
 
 // The whole scan of a small grid in one CTA: one launch less than the two above where launches are most of the time.
@@ -531,7 +534,8 @@ __global__ void __launch_bounds__(1024) k_scan_small(const uint4* __restrict__ r
                                                      const uint32_t* __restrict__ mccnt, int R,
                                                      unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
                                                      unsigned long long* __restrict__ totals,
-                                                     unsigned long long* __restrict__ publish)
+                                                     unsigned long long* __restrict__ publish,
+                                                     unsigned long long* __restrict__ kept)
 {
     constexpr int NC = ScanComps<SM>::n, PER = kScanSmallPer;
     __shared__ uint32_t s_w[NC][32];
@@ -604,7 +608,7 @@ __global__ void __launch_bounds__(1024) k_scan_small(const uint4* __restrict__ r
             totals[4] = run[0];
             totals[5] = e2;
         }
-        scan_publish(totals, V, run[1], m, publish);
+        scan_publish(totals, V, run[1], m, publish, kept);
     }
 }
 
@@ -630,7 +634,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_final_batch(const BatchReq* _
     const int blk = (int)(blockIdx.x - __ldg(&first[q]));
     if (blk >= d->nseg) return;
     scan_final_block<kScanFE>(d->rowcnt, nullptr, d->g.R, d->part, d->nseg, d->starts, d->row4,
-                              d->totals, nullptr, blk);
+                              d->totals, nullptr, nullptr, blk);
 }
 
 // vfirst[q] = the vertices of requests list[0 .. q-1] whose meshes hold their counts (one CTA of 1024 threads,
@@ -905,12 +909,13 @@ template <int SM>
 static void scan_launch(const Grid& g, const CountPlan& p, FeBuffers& b, cudaStream_t s, unsigned long long* publish)
 {
     if (g.R <= kScanSmall && g.nx <= (1 << 15)) {  // their triangles stay below 2^32
-        launch_after(k_scan_small<SM>, 1, 1024, 0, s, b.rowcnt, b.mccnt, (int)g.R, b.starts, b.row4, b.totals, publish);
+        launch_after(k_scan_small<SM>, 1, 1024, 0, s, b.rowcnt, b.mccnt, (int)g.R, b.starts, b.row4, b.totals, publish,
+                     b.kept);
         return;
     }
     launch_after(k_scan_partial<SM>, p.nseg, kThreads, 0, s, b.rowcnt, b.mccnt, g.R, b.part, p.nseg);
     launch_after(k_scan_final<SM>, p.nseg, kThreads, 0, s, b.rowcnt, b.mccnt, g.R, b.part, p.nseg, b.starts, b.row4,
-                 b.totals, publish);
+                 b.totals, publish, b.kept);
 }
 
 void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,

@@ -22,8 +22,9 @@ struct FeBuffers {
     uint32_t* mccnt = nullptr;             // R      MC vertices per cell row
     unsigned long long* starts = nullptr;  // 4*R    per row: first vertex, triangle, MC vertex (or y, z cuts)
     unsigned long long* part = nullptr;    // 4*nseg scan segment totals
-    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, kept status, work counter
+    unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, -, work counter
     uint32_t* bits = nullptr;              // R*W    bit rows
+    unsigned long long* kept = nullptr;    // 1      device status of the calls that publish (count_status)
     uint32_t* fe2mc = nullptr;             // >= V   FE vertex index -> MC index
 };
 
@@ -102,19 +103,18 @@ CountRows count_rows_plan(const Grid& g, int nsm, int sample_bytes, bool aligned
 GenPlan gen_plan(const Grid& g, int nsm);
 
 // passes 1-3
-// The device status of a count: totals[3], zeroed before it, or with zero_status off a word that the scan's publish
-// leaves at zero and nothing else writes (an extraction that does not publish leaves its own status behind).
-constexpr int kStatusKept = 6;
+// The device status of a count: totals[3], zeroed before it, or with zero_status off the context's own word, which is
+// zero from its creation on, the scan's publish leaves at zero and nothing else writes.
 inline unsigned long long* count_status(const FeBuffers& b, bool zero_status, cudaStream_t s)
 {
     if (zero_status) cudaMemsetAsync(b.totals + 3, 0, sizeof(unsigned long long), s);
-    return b.totals + (zero_status ? 3 : kStatusKept);
+    return zero_status ? b.totals + 3 : b.kept;
 }
 void launch_count(const float* vol, const Grid& g, float iso, const CaseTables* cases, bool mc,
                   const CountPlan& p, FeBuffers& b, cudaStream_t s, bool zero_status = true);
 enum ScanMode { kScanFE = 0, kScanMC = 1, kScanDup = 2 };
 // Row starts and totals; the work counter of pass 4 (totals[7]) zeroed.  publish (device-visible host memory, or null):
-// the totals and the device status are also written there, and the status is zero again for the next count.
+// the totals and the context's status word are also written there, and that word is zero again for the next count.
 void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,
                  unsigned long long* publish = nullptr);
 // totals and the starts of rows rlo / rhi into out[0..8] (device-visible host memory)
