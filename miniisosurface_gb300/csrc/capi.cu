@@ -52,39 +52,42 @@ struct SlabCounts {
     unsigned long long lo[3], hi[3], tot[3];
 };
 
-// Enqueues the count of the window and the copies of its totals and row
-// starts into h[0..8] (pinned).
 // The slab-count read-back buffer: pinned host memory that kernels write.
 iso_status ensure_h_slab(iso_ctx* ctx)
 {
     if (ctx->h_slab) return ISO_OK;
-    ISO_CUDA(ctx, cudaHostAlloc(&ctx->h_slab, 18 * sizeof(unsigned long long), cudaHostAllocMapped));
+    ISO_CUDA(ctx, cudaHostAlloc(&ctx->h_slab, 2 * kSlabWords * sizeof(unsigned long long), cudaHostAllocMapped));
     ISO_CUDA(ctx, cudaHostGetDevicePointer(reinterpret_cast<void**>(&ctx->h_slab_dev), ctx->h_slab, 0));
     return ISO_OK;
 }
 
+// Enqueues the count of the window, which writes its totals and the device status into h[0..3] (within ctx->h_slab),
+// and its starts at planes k0 and k1 into h[4..9].
 iso_status slab_count_enqueue(iso_ctx* ctx, iso_algorithm algo, const float* vol, const Grid& g, int64_t k0,
                               int64_t k1, float iso, const Plans& pl, FeBuffers& b, cudaStream_t s,
                               unsigned long long* h)
 {
     PassMarks pm(ctx, s);
-    enqueue_count(ctx, algo, vol, g, iso, pl, b, s, pm);
+    unsigned long long* d = ctx->h_slab_dev + (h - ctx->h_slab);  // kernels write it through the device address
+    enqueue_count(ctx, algo, vol, g, iso, pl, b, s, pm, d);
     ISO_CUDA(ctx, cudaGetLastError());
-    // h lies in ctx->h_slab; the kernel writes it through the device address
     const long long rlo = (long long)(k0 - g.kr) * g.ny, rhi = (long long)(k1 - g.kr) * g.ny;
-    iso::launch_slab_readback(b, g, rlo, rhi, rlo > 0, k1 < g.nz, ctx->h_slab_dev + (h - ctx->h_slab), s);
+    iso::launch_slab_readback(b, g, rlo, rhi, rlo > 0, k1 < g.nz, d + 4, s);
     ISO_CUDA(ctx, cudaGetLastError());
     return ISO_OK;
 }
 
-// The counts copied by slab_count_enqueue, once they have landed.
-void slab_count_read(const Grid& g, int64_t k0, int64_t k1, const unsigned long long* h, SlabCounts& c)
+// The counts written by slab_count_enqueue, once they have landed.
+iso_status slab_count_read(iso_ctx* ctx, const Grid& g, int64_t k0, int64_t k1, const unsigned long long* h,
+                           SlabCounts& c)
 {
     for (int a = 0; a < 3; ++a) {
         c.tot[a] = h[a];
-        c.lo[a] = k0 - g.kr > 0 ? h[3 + a] : 0;
-        c.hi[a] = k1 < g.nz ? h[6 + a] : h[a];
+        c.lo[a] = k0 - g.kr > 0 ? h[4 + a] : 0;
+        c.hi[a] = k1 < g.nz ? h[7 + a] : h[a];
     }
+    int64_t v, t;
+    return finish_counts(ctx, nullptr, (long long)h[0], (long long)h[1], (long long)h[3], &v, &t);
 }
 
 iso_status slab_count(iso_ctx* ctx, iso_algorithm algo, const float* vol, const Grid& g, int64_t k0, int64_t k1,
@@ -95,8 +98,7 @@ iso_status slab_count(iso_ctx* ctx, iso_algorithm algo, const float* vol, const 
     st = slab_count_enqueue(ctx, algo, vol, g, k0, k1, iso, pl, b, s, ctx->h_slab);
     if (st != ISO_OK) return st;
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
-    slab_count_read(g, k0, k1, ctx->h_slab, c);
-    return ISO_OK;
+    return slab_count_read(ctx, g, k0, k1, ctx->h_slab, c);
 }
 
 // Pass 4 of slab [k0, k1) into the device mesh `out` (the slab's rows),
@@ -348,7 +350,7 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
         FeBuffers b;
         int k0, k1;
     } run[2];
-    const size_t ev_cnt = ev_out + 2;  // 2 events: counts of slab q landed in h_slab + 9 * (q & 1)
+    const size_t ev_cnt = ev_out + 2;  // 2 events: counts of slab q landed in h_slab + kSlabWords * (q & 1)
     const size_t ev_scr = ev_cnt + 2;  // 2 events: slab q generated, scratch set q & 1 free again
     auto start_count = [&](int q) -> iso_status {
         SlabRun& r = run[q & 1];
@@ -366,7 +368,7 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
             (q & 1) ? ensure_scratch_b(ctx, r.g, r.pl.cp, r.b, sc) : ensure_scratch(ctx, r.g, r.pl.cp, r.b, sc);
         if (e != ISO_OK) return e;
         e = slab_count_enqueue(ctx, algo, window(q), r.g, r.k0, r.k1, isoval, r.pl, r.b, sc,
-                               ctx->h_slab + 9 * (q & 1));
+                               ctx->h_slab + kSlabWords * (q & 1));
         if (e != ISO_OK) return e;
         ISO_CUDA(ctx, cudaEventRecord(sync_event(ctx, ev_cnt + (q & 1)), sc));
         return ISO_OK;
@@ -386,7 +388,8 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
         ISO_CUDA(ctx, cudaEventSynchronize(sync_event(ctx, ev_cnt + (q & 1))));
         ISO_CUDA(ctx, cudaStreamWaitEvent(s, sync_event(ctx, ev_cnt + (q & 1)), 0));
         SlabCounts c;
-        slab_count_read(g, k0, k1, ctx->h_slab + 9 * (q & 1), c);
+        st = slab_count_read(ctx, g, k0, k1, ctx->h_slab + kSlabWords * (q & 1), c);
+        if (st != ISO_OK) break;
         const long long Vq = (long long)(c.hi[mc ? 2 : 0] - c.lo[mc ? 2 : 0]), Tq = (long long)(c.hi[1] - c.lo[1]);
         const long long top = V + (mc ? Vq : (long long)c.tot[0]);  // largest id the slab references
         if (out->index_bytes == 4 && top > 0xffffffffll) {
@@ -694,9 +697,8 @@ iso_status iso_count_device(iso_ctx* ctx, iso_algorithm algo, const float* volum
     enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm, ctx->h_totals);
     ISO_CUDA(ctx, cudaGetLastError());
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
-    *n_points = (int64_t)ctx->h_totals[0];
-    *n_tris = (int64_t)ctx->h_totals[1];
-    return ISO_OK;
+    return finish_counts(ctx, nullptr, (long long)ctx->h_totals[0], (long long)ctx->h_totals[1],
+                         (long long)ctx->h_totals[3], n_points, n_tris);
 }
 
 // sync: result_host is the context's own h_totals, which the scan writes itself, and the call is not captured.
@@ -803,12 +805,11 @@ static iso_status extract_host_impl(iso_ctx* ctx, iso_algorithm algo, const void
     st = ensure_scratch(ctx, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     PassMarks pm(ctx, s);
-    enqueue_count(ctx, algo, ctx->d_volume, g, isoval, pl, b, s, pm);
+    enqueue_count(ctx, algo, ctx->d_volume, g, isoval, pl, b, s, pm, ctx->h_totals);
     ISO_CUDA(ctx, cudaGetLastError());
-    ISO_CUDA(ctx, cudaMemcpyAsync(ctx->h_totals, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
     const long long V = (long long)ctx->h_totals[0], T = (long long)ctx->h_totals[1];
-    st = finish_counts(ctx, out, V, T, 0, &out->n_points, &out->n_tris);
+    st = finish_counts(ctx, out, V, T, (long long)ctx->h_totals[3], &out->n_points, &out->n_tris);
     if (st != ISO_OK) return st;
     // device output staging, grown on demand
     if (V > ctx->d_cap_points || T > ctx->d_cap_tris || out->index_bytes != ctx->d_index_bytes) {
@@ -847,9 +848,8 @@ static iso_status extract_host_impl(iso_ctx* ctx, iso_algorithm algo, const void
     if (T > 0) {
         ISO_CUDA(ctx, cudaMemcpyAsync(out->tris, dm.tris, (size_t)T * 3 * out->index_bytes, cudaMemcpyDeviceToHost, s));
     }
-    ISO_CUDA(ctx, cudaMemcpyAsync(ctx->h_totals, b.totals, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     ISO_CUDA(ctx, cudaStreamSynchronize(s));
-    return finish_counts(ctx, out, V, T, (long long)ctx->h_totals[3], &out->n_points, &out->n_tris);
+    return ISO_OK;
 }
 
 iso_status iso_extract_host(iso_ctx* ctx, iso_algorithm algo, const float* volume, const iso_grid* grid,

@@ -36,8 +36,8 @@ struct iso_ctx {
     int d_index_bytes = 0;
     unsigned long long* h_totals = nullptr;  // pinned, 4 entries
     unsigned long long* d_status = nullptr;  // device status of the publishing calls, one word, zero between them
-    unsigned long long* h_slab = nullptr;    // pinned and mapped, 2 x 9 entries (slab counts)
-    unsigned long long* h_slab_dev = nullptr;  // its device address (written by k_slab_readback)
+    unsigned long long* h_slab = nullptr;    // pinned and mapped, 2 x kSlabWords entries (slab counts)
+    unsigned long long* h_slab_dev = nullptr;  // its device address (the scan and k_slab_readback write it)
     void* scratch_b = nullptr;               // second scratch set (streamed path: the next slab's counts)
     size_t scratch_b_bytes = 0;
     void* d_typed = nullptr;                 // typed volume samples before conversion
@@ -91,6 +91,8 @@ struct iso_ctx {
 };
 
 namespace capi {
+
+constexpr int kSlabWords = 10;  // a slab's totals and status, its starts at both planes
 
 inline iso_status cuda_fail(iso_ctx* ctx, cudaError_t e, const char* what)
 {

@@ -117,7 +117,7 @@ enum ScanMode { kScanFE = 0, kScanMC = 1, kScanDup = 2 };
 // the totals and the context's status word are also written there, and that word is zero again for the next count.
 void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,
                  unsigned long long* publish = nullptr);
-// totals and the starts of rows rlo / rhi into out[0..8] (device-visible host memory)
+// the starts of rows rlo / rhi into out[0..5] (device-visible host memory)
 void launch_slab_readback(const FeBuffers& b, const Grid& g, long long rlo, long long rhi, bool has_lo, bool has_hi,
                           unsigned long long* out, cudaStream_t s);
 // Marching Cubes in two passes (rows of up to 32 words, whole windows): owned

@@ -1,0 +1,96 @@
+// A count pass that gave up leaves a status behind: every call that reads counts has to report it, and the next one
+// has to run again.  The status is set by hand in the context's word before each call (no wait runs out here).
+#include <cmath>
+#include <cstdio>
+#include <functional>
+
+#include "../../miniisosurface_gb300/csrc/capi_internal.h"
+
+static int failures = 0;
+
+static void expect(const char* what, long long got, long long want)
+{
+    if (got == want) return;
+    std::printf("%s: %lld, expected %lld\n", what, got, want);
+    ++failures;
+}
+
+int main()
+{
+    iso_ctx* ctx = nullptr;
+    if (iso_ctx_create(0, &ctx) != ISO_OK) {
+        std::printf("no context\n");
+        return 2;
+    }
+    // rows read by the bulk-copy count and long ones by the row-wise kernels; enough planes for the streamed host path
+    const int64_t dims[3][3] = {{40, 33, 27}, {1100, 5, 4}, {20, 9, 140}};
+    for (const auto& d : dims) {
+        iso_grid g{};
+        const int64_t n = d[0] * d[1] * d[2];
+        for (int a = 0; a < 3; ++a) {
+            g.dims[a] = d[a];
+            g.spacing[a] = 1.f;
+        }
+        std::vector<float> host(n);
+        std::vector<uint8_t> bytes(n);
+        for (int64_t q = 0; q < n; ++q) {
+            bytes[q] = (uint8_t)((q * q / 7 + q) % 11);
+            host[q] = bytes[q];
+        }
+        float* vol = nullptr;
+        uint8_t* typed = nullptr;
+        const int64_t capV = 3 * n, capT = 5 * n;
+        iso_mesh dev{}, hst{};
+        std::vector<float> hp(3 * capV), hn(3 * capV);
+        std::vector<uint32_t> ht(3 * capT);
+        hst.points = hp.data(), hst.normals = hn.data(), hst.tris = ht.data();
+        if (cudaMalloc(&vol, n * 4) != cudaSuccess || cudaMalloc(&typed, n) != cudaSuccess ||
+            cudaMalloc(&dev.points, capV * 12) != cudaSuccess || cudaMalloc(&dev.normals, capV * 12) != cudaSuccess ||
+            cudaMalloc(&dev.tris, capT * 12) != cudaSuccess)
+            return 2;
+        dev.index_bytes = hst.index_bytes = 4;
+        dev.cap_points = hst.cap_points = capV;
+        dev.cap_tris = hst.cap_tris = capT;
+        cudaMemcpy(vol, host.data(), n * 4, cudaMemcpyHostToDevice);
+        cudaMemcpy(typed, bytes.data(), n, cudaMemcpyHostToDevice);
+        const int64_t k1 = d[2] / 2;
+        int64_t V = 0, T = 0;
+        for (iso_algorithm algo : {ISO_FLYING_EDGES, ISO_MARCHING_CUBES, ISO_MC_DUPFREE}) {
+            if (algo == ISO_MC_DUPFREE && d[0] > 1024) continue;
+            struct Call {
+                const char* name;
+                std::function<iso_status()> run;
+            };
+            std::vector<Call> calls = {
+                {"count", [&] { return iso_count_device(ctx, algo, vol, &g, 5.5f, &V, &T, nullptr); }},
+                {"extract", [&] { return iso_extract_device(ctx, algo, vol, &g, 5.5f, &dev, nullptr); }},
+                {"typed", [&] { return iso_extract_device_typed(ctx, algo, typed, ISO_UINT8, &g, 5.5f, &dev, nullptr); }},
+                {"host", [&] { return iso_extract_host(ctx, algo, host.data(), &g, 5.5f, &hst, nullptr); }}};
+            if (algo != ISO_MC_DUPFREE && d[0] <= 1024) {
+                calls.push_back({"slab count",
+                                 [&] { return iso_count_slab(ctx, algo, vol, &g, 0, k1, 5.5f, &V, &T, nullptr); }});
+                calls.push_back({"slab", [&] {
+                                     return iso_extract_slab(ctx, algo, vol, &g, 0, k1, 5.5f, 0, 0, &dev, nullptr);
+                                 }});
+            }
+            for (const Call& c : calls) {
+                char what[96];
+                std::snprintf(what, sizeof what, "%s, algorithm %d, row of %lld", c.name, (int)algo, (long long)d[0]);
+                expect(what, c.run(), ISO_OK);
+                const unsigned long long one = 1;
+                cudaMemcpy(ctx->d_status, &one, sizeof one, cudaMemcpyHostToDevice);
+                cudaDeviceSynchronize();
+                expect(what, c.run(), ISO_ERR_TIMEOUT);
+                expect(what, c.run(), ISO_OK);
+            }
+        }
+        cudaFree(vol);
+        cudaFree(typed);
+        cudaFree(dev.points);
+        cudaFree(dev.normals);
+        cudaFree(dev.tris);
+    }
+    iso_ctx_destroy(ctx);
+    std::printf("%d failures\n", failures);
+    return failures ? 1 : 0;
+}
