@@ -396,7 +396,7 @@ __device__ __forceinline__ void scan_publish(unsigned long long* __restrict__ to
         publish[0] = v;
         publish[1] = t;
         publish[2] = m;
-        publish[3] = *kept;
+        publish[3] = totals[3] = *kept;  // pass 4 looks at totals[3]
         *kept = 0;
     }
 }
@@ -647,8 +647,7 @@ __global__ void __launch_bounds__(1024) k_batch_vfirst(const BatchReq* __restric
     const int per = (m + 1023) / 1024, q0 = t * per, q1 = min(m, q0 + per);
     auto verts = [&](int q) -> unsigned long long {
         const BatchReq* d = reqs + __ldg(&list[q]);
-        const unsigned long long v = d->totals[0], tr = d->totals[1];
-        return ((long long)v <= d->capV && (long long)tr <= d->capT) ? v : 0ull;
+        return mesh_holds(d->totals, d->capV, d->capT) ? d->totals[0] : 0ull;
     };
     unsigned long long mine = 0;
     for (int q = q0; q < q1; ++q) mine += verts(q);
@@ -720,7 +719,7 @@ __global__ void __launch_bounds__(1024) k_batch_place(BatchReq* __restrict__ req
         BatchReq* d = reqs + __ldg(&list[q]);
         const unsigned long long V = d->totals[0], T = d->totals[1];
         const bool ok = vat + V <= (unsigned long long)o.cap_points && tat + T <= (unsigned long long)o.cap_tris &&
-                        (o.index_bytes == 8 || V <= 0xffffffffull);
+                        (o.index_bytes == 8 || V <= 0xffffffffull) && d->totals[3] == 0ull;
         d->points = o.points + 3 * vat;
         d->normals = o.normals + 3 * vat;
         d->tris = static_cast<char*>(o.tris) + 3 * tat * (unsigned long long)o.index_bytes;

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells(
     // Caller grows buffers.  Past this check every record slot and triangle index written below lies
     // under the totals, because the count pass derives the counts and starts from the same bit words
     // with the same masks; the writes are not checked one by one.
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
+    if (!mesh_holds(totals, capV, capT)) return;
     const uint32_t ws = (threadIdx.x >> 5) * (uint32_t)ws_bytes;
     const GenLane ln = gen_lane(g, RPW > 0 ? RPW : rpw, gen_extra_slot(RPW));
     for (uint32_t item; (item = gen_take(work)) < nitems;) {
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(32 * kGenBatchWarps, 2) k_gen_cells_batch(
     for (uint32_t item; (item = gen_take(work)) < nitems;) {
         const int q = batch_find(first, m, item);
         const BatchReq* d = reqs + __ldg(&list[q]);
-        if ((long long)d->totals[0] > d->capV || (long long)d->totals[1] > d->capT) continue;
+        if (!mesh_holds(d->totals, d->capV, d->capT)) continue;
         if (item - __ldg(&first[q]) >= (uint32_t)d->gen_ngroups * (uint32_t)d->gen_nkc) continue;  // past its items
         const Grid g = d->g;
         unsigned long long* out = s_out[threadIdx.x >> 5];

@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(kThreads) k_gen_rows(
 {
     __shared__ SharedCases s_cases;
     stage_cases(s_cases, cases, false);
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;  // caller grows buffers
+    if (!mesh_holds(totals, capV, capT)) return;  // caller grows buffers
 
     const int lane = threadIdx.x & 31;
     const int lig = lane & (G - 1), grp = lane / G;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads) k_mc_vertices_rows(
 {
     __shared__ SharedCases s_cases;
     stage_cases(s_cases, cases, true);
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
+    if (!mesh_holds(totals, capV, capT)) return;
 
     const int lane = threadIdx.x & 31;
     const int lig = lane & (G - 1), grp = lane / G;

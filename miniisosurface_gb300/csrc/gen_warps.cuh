@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, kGenCtasPerSm) k_gen_warps(
         s_tris[c] = cases->tris[c];
     }
     __syncthreads();  // the only CTA barrier: from here on every warp runs alone
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;  // caller grows buffers
+    if (!mesh_holds(totals, capV, capT)) return;  // caller grows buffers
     const unsigned long long dupY = totals[4];              // all x cuts
     const unsigned long long dupZ = totals[4] + totals[5];  // all x and y cuts
 

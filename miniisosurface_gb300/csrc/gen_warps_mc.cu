@@ -108,7 +108,7 @@ __global__ void k_mc_remap(IndexT* __restrict__ tris, const uint32_t* __restrict
                            const unsigned long long* __restrict__ totals, long long capV, long long capT)
 {
     wait_for_previous();
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
+    if (!mesh_holds(totals, capV, capT)) return;
     const unsigned long long n = 3ull * totals[1];
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const unsigned long long t0 = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -427,6 +427,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Whether pass 4 may write: the mesh holds the counts, and the counts belong to this volume.  After a count pass whose
+// wait ran out (totals[3]) some rows hold the bits and counts of an earlier call, and with them places outside the mesh.
+__device__ __forceinline__ bool mesh_holds(const unsigned long long* totals, long long capV, long long capT)
+{
+    return (long long)totals[0] <= capV && (long long)totals[1] <= capT && totals[3] == 0ull;
+}
+
 // First vertex (comp 0), triangle (1) or MC vertex (2) of grid row r =
 // k*ny + j, from the scanned starts[3][R].
 // Window row r (see Grid); add[comp] shifts the window's numbering to the

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, vertex_ctas_per_sm(MC))
 {
     wait_for_previous();
     next_may_start();
-    if ((long long)totals[0] > capV || (long long)totals[1] > capT) return;
+    if (!mesh_holds(totals, capV, capT)) return;
     auto first = [&](int p) { return p < g.ke ? starts[COMP * g.R + (long long)(p - g.kr) * g.ny] : totals[COMP]; };
     const unsigned long long n = first(kend) - first(kbeg);
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;

@@ -1,5 +1,6 @@
-// A count pass that gave up leaves a status behind: every call that reads counts has to report it, and the next one
-// has to run again.  The status is set by hand in the context's word before each call (no wait runs out here).
+// A count pass that gave up leaves a status behind: every call that reads counts has to report it and to leave the
+// mesh alone (rows that were not counted hold an earlier call's places), and the next call has to run again.  The status
+// is set by hand in the context's word before each call (no wait runs out here).
 #include <cmath>
 #include <cstdio>
 #include <functional>
@@ -13,6 +14,14 @@ static void expect(const char* what, long long got, long long want)
     if (got == want) return;
     std::printf("%s: %lld, expected %lld\n", what, got, want);
     ++failures;
+}
+
+// Bytes at p that are not 0xab.
+static long long written(const void* p, size_t n)
+{
+    std::vector<unsigned char> b(n);
+    cudaMemcpy(b.data(), p, n, cudaMemcpyDeviceToHost);
+    return (long long)(n - std::count(b.begin(), b.end(), 0xab));
 }
 
 int main()
@@ -79,8 +88,13 @@ int main()
                 expect(what, c.run(), ISO_OK);
                 const unsigned long long one = 1;
                 cudaMemcpy(ctx->d_status, &one, sizeof one, cudaMemcpyHostToDevice);
+                cudaMemset(dev.points, 0xab, capV * 12);
+                cudaMemset(dev.normals, 0xab, capV * 12);
+                cudaMemset(dev.tris, 0xab, capT * 12);
                 cudaDeviceSynchronize();
                 expect(what, c.run(), ISO_ERR_TIMEOUT);
+                expect(what, written(dev.points, capV * 12) + written(dev.normals, capV * 12) +
+                                 written(dev.tris, capT * 12), 0);
                 expect(what, c.run(), ISO_OK);
             }
         }
