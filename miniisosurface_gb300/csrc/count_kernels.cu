@@ -324,7 +324,7 @@ struct ScanComps {
 };
 
 template <int SM>
-__device__ __forceinline__ void load_counts(const uint4* __restrict__ rowcnt, const uint32_t* __restrict__ mccnt,
+__device__ __forceinline__ void load_counts(const uint4* rowcnt, const uint32_t* mccnt,
                                             long long R, long long b, uint32_t (&v)[4][kScanPer],
                                             unsigned long long (&s)[4])
 {
@@ -332,14 +332,14 @@ __device__ __forceinline__ void load_counts(const uint4* __restrict__ rowcnt, co
 #pragma unroll
     for (int q = 0; q < kScanPer; ++q) {
         const bool ok = b + q < R;
-        const uint4 c = ok ? __ldg(&rowcnt[b + q]) : make_uint4(0, 0, 0, 0);
+        const uint4 c = ok ? load_written(rowcnt + b + q) : make_uint4(0, 0, 0, 0);
         if (SM == kScanDup) {
             v[0][q] = c.x;
             v[2][q] = c.y;
             v[3][q] = c.z;
         } else {
             v[0][q] = c.x + c.y + c.z;
-            v[2][q] = (SM == kScanMC && ok) ? __ldg(&mccnt[b + q]) : 0u;
+            v[2][q] = (SM == kScanMC && ok) ? load_written(mccnt + b + q) : 0u;
             v[3][q] = 0u;
         }
         v[1][q] = c.w;
@@ -350,8 +350,8 @@ __device__ __forceinline__ void load_counts(const uint4* __restrict__ rowcnt, co
 
 // Segment blk of the scan: its totals into part[a * nseg + blk].
 template <int SM>
-__device__ __forceinline__ void scan_partial_block(const uint4* __restrict__ rowcnt,
-                                                   const uint32_t* __restrict__ mccnt, long long R,
+__device__ __forceinline__ void scan_partial_block(const uint4* rowcnt,
+                                                   const uint32_t* mccnt, long long R,
                                                    unsigned long long* __restrict__ part, int nseg, int blk)
 {
     constexpr int NC = ScanComps<SM>::n;
@@ -375,8 +375,8 @@ __device__ __forceinline__ void scan_partial_block(const uint4* __restrict__ row
 }
 
 template <int SM>
-__global__ void __launch_bounds__(kThreads) k_scan_partial(const uint4* __restrict__ rowcnt,
-                                                           const uint32_t* __restrict__ mccnt, long long R,
+__global__ void __launch_bounds__(kThreads) k_scan_partial(const uint4* rowcnt,
+                                                           const uint32_t* mccnt, long long R,
                                                            unsigned long long* __restrict__ part, int nseg)
 {
     wait_for_previous();
@@ -411,9 +411,9 @@ __device__ __forceinline__ void store_sector(unsigned long long* p, unsigned lon
 
 // Segment blk: the starts of its rows from the segments' totals; segment 0 also writes the totals.
 template <int SM>
-__device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcnt,
-                                                 const uint32_t* __restrict__ mccnt, long long R,
-                                                 const unsigned long long* __restrict__ part, int nseg,
+__device__ __forceinline__ void scan_final_block(const uint4* rowcnt,
+                                                 const uint32_t* mccnt, long long R,
+                                                 const unsigned long long* part, int nseg,
                                                  unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
                                                  unsigned long long* __restrict__ totals,
                                                  unsigned long long* __restrict__ publish,
@@ -426,7 +426,7 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
     if (warp < NC) {  // warp a: the segments before this one and all of them, for component a
         unsigned long long b = 0, tot = 0;
         for (int q = lane; q < nseg; q += 32) {
-            const unsigned long long x = part[warp * nseg + q];
+            const unsigned long long x = load_written(part + warp * nseg + q);
             if (q < blk) b += x;
             tot += x;
         }
@@ -509,9 +509,9 @@ __device__ __forceinline__ void scan_final_block(const uint4* __restrict__ rowcn
 }
 
 template <int SM>
-__global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* __restrict__ rowcnt,
-                                                         const uint32_t* __restrict__ mccnt, long long R,
-                                                         const unsigned long long* __restrict__ part, int nseg,
+__global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* rowcnt,
+                                                         const uint32_t* mccnt, long long R,
+                                                         const unsigned long long* part, int nseg,
                                                          unsigned long long* __restrict__ starts,
                                                          uint4* __restrict__ row4,
                                                          unsigned long long* __restrict__ totals,
@@ -530,8 +530,8 @@ constexpr int kScanSmallPer = 4;
 constexpr long long kScanSmall = 1024ll * kScanSmallPer;
 
 template <int SM>
-__global__ void __launch_bounds__(1024) k_scan_small(const uint4* __restrict__ rowcnt,
-                                                     const uint32_t* __restrict__ mccnt, int R,
+__global__ void __launch_bounds__(1024) k_scan_small(const uint4* rowcnt,
+                                                     const uint32_t* mccnt, int R,
                                                      unsigned long long* __restrict__ starts, uint4* __restrict__ row4,
                                                      unsigned long long* __restrict__ totals,
                                                      unsigned long long* __restrict__ publish,
@@ -549,12 +549,12 @@ __global__ void __launch_bounds__(1024) k_scan_small(const uint4* __restrict__ r
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
         const int r = r0 + 32 * q;
-        const uint4 c = r < R ? __ldg(&rowcnt[r]) : make_uint4(0u, 0u, 0u, 0u);
+        const uint4 c = r < R ? load_written(rowcnt + r) : make_uint4(0u, 0u, 0u, 0u);
         cx[q] = c.x;
         cxy[q] = c.x + c.y;
         v[0][q] = SM == kScanDup ? c.x : c.x + c.y + c.z;
         v[1][q] = c.w;
-        if (NC > 2) v[NC > 2 ? 2 : 0][q] = SM == kScanDup ? c.y : (r < R ? __ldg(&mccnt[r]) : 0u);
+        if (NC > 2) v[NC > 2 ? 2 : 0][q] = SM == kScanDup ? c.y : (r < R ? load_written(mccnt + r) : 0u);
         if (NC > 3) v[NC > 3 ? 3 : 0][q] = c.z;
 #pragma unroll
         for (int a = 0; a < NC; ++a) sum[a] += v[a][q];

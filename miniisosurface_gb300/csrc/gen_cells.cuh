@@ -182,7 +182,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
                                                const GenCellTables<MODE>& tabs, const uint32_t* __restrict__ bits,
                                                const Grid& g, const GenLane& ln, int rpw_, const GenCols& cols, int ngroups,
                                                int kbeg, int kend, int kemit, unsigned long long vbase,
-                                               unsigned long long tbase, const uint4* __restrict__ row4,
+                                               unsigned long long tbase, const uint4* row4,
                                                const RowStarts& rs, const Out& out, uint32_t* __restrict__ fe2mc, int reverse)
 {
     constexpr bool OWNS = GenCellTables<MODE>::OWNS, TRIS = GenCellTables<MODE>::TRIS;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
     for (int s = 0; s < NS; ++s) {
         wp[s] = zb[s] = 0u;
         w[s] = s * rpw < nrow ? __ldg(bp + s * RW) : 0u;
-        q[s] = s * rpw < nrow ? __ldg(qp + s * rpw) : make_uint4(0u, 0u, 0u, 0u);
+        q[s] = s * rpw < nrow ? load_written(qp + s * rpw) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) pand[s] = por[s] = 0u;
@@ -231,9 +231,9 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
         const uint32_t par = (uint32_t)(p & 1) * 8u, kpar = par ^ 8u;  // this plane's copy, the plane before's
         const bool cells = p > kb;
         unsigned long long tcur = tnext, mcur = mnext, xw = 0ull;
-        if (TRIS) tnext = __ldg(sp + rs.R) + rs.add[1];
-        if (OWNS) mnext = __ldg(sp + 2 * rs.R) + rs.add[2];
-        if (WIDE) xw = __ldg(sp) + rs.add[0];
+        if (TRIS) tnext = load_written(sp + rs.R) + rs.add[1];
+        if (OWNS) mnext = load_written(sp + 2 * rs.R) + rs.add[2];
+        if (WIDE) xw = load_written(sp) + rs.add[0];
         uint32_t act[S];
         {
             uint32_t wn[NS];
@@ -310,7 +310,7 @@ __device__ __forceinline__ void gen_cells_item(uint32_t item, unsigned char* s_r
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
                     w[s] = s * rpw < nrow ? __ldg(bp + s * RW) : 0u;
-                    q[s] = s * rpw < nrow ? __ldg(qp + s * rpw) : make_uint4(0u, 0u, 0u, 0u);
+                    q[s] = s * rpw < nrow ? load_written(qp + s * rpw) : make_uint4(0u, 0u, 0u, 0u);
                 }
             }
         }
@@ -468,7 +468,7 @@ template <typename IndexT, int MODE, int RPW>
 __global__ void __launch_bounds__(32 * kGenMaxWarps, 2) k_gen_cells(
     const uint32_t* __restrict__ bits, Grid g, int rpw, GenCols cols, int ngroups, uint32_t nitems, int kbeg, int kend, int kemit,
     unsigned long long vbase, unsigned long long tbase, int ws_bytes, const CaseTables* __restrict__ cases,
-    const uint4* __restrict__ row4, RowStarts rs, const unsigned long long* __restrict__ totals,
+    const uint4* row4, RowStarts rs, const unsigned long long* totals,
     unsigned int* __restrict__ work, long long capV, long long capT, float* __restrict__ points,
     IndexT* __restrict__ tris, uint32_t* __restrict__ fe2mc, int reverse)
 {

@@ -427,6 +427,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A value that the kernel before wrote, read after wait_for_previous: by the coherent path and in program order.  __ldg
+// and const __restrict__ parameters promise memory that nothing writes while the kernel runs, which does not hold for a
+// kernel brought in beside its predecessor: such a load may come from a cache that the predecessor's stores do not
+// reach, and the compiler may move it above the wait.  What the kernels before the predecessor wrote is complete before
+// this one starts (every thread of the predecessor waits before it lets its successor in): the vertex kernel reads the
+// scan's totals and starts as read-only memory (their other form spilled: 512^3 166 us -> 188).
+__device__ __forceinline__ uint32_t load_written(const uint32_t* p)
+{
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned long long load_written(const unsigned long long* p)
+{
+    unsigned long long v;
+    asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 load_written(const uint4* p)
+{
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // Whether pass 4 may write: the mesh holds the counts, and the counts belong to this volume.  After a count pass whose
 // wait ran out (totals[3]) some rows hold the bits and counts of an earlier call, and with them places outside the mesh.
 __device__ __forceinline__ bool mesh_holds(const unsigned long long* totals, long long capV, long long capT)
