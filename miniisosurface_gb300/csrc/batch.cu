@@ -205,7 +205,7 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
     f.scratch_at.resize(nf);
     for (int d = 0; d < nf; ++d) {
         f.scratch_at[d] = at;
-        at += align256(scratch_size(items[fz[d]].g, items[fz[d]].pl.cp));
+        at += align256(scratch_size(ISO_FLYING_EDGES, items[fz[d]].g, items[fz[d]].pl.cp));
     }
     f.bytes = at;
     return f;
@@ -222,7 +222,7 @@ void fill_fused(iso_ctx* ctx, const FusedPlan& f, const iso_mesh* out, const std
         const int r = f.reqs[d];
         const BatchItem& it = items[r];
         FeBuffers b;
-        carve(base + f.scratch_at[d], it.g, it.pl.cp, b);
+        carve(base + f.scratch_at[d], ISO_FLYING_EDGES, it.g, it.pl.cp, b);
         iso::BatchReq x = f.proto[d];
         x.rowcnt = b.rowcnt;
         x.row4 = b.row4;
@@ -320,7 +320,8 @@ BatchLayout plan_batch(const iso_request* req, const iso_mesh* out, int64_t n, s
         const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
         items[r].lane = l;
         load[l] += cells(r);
-        scratch[l] = std::max(scratch[l], scratch_size(items[r].g, items[r].pl.cp));
+        scratch[l] = std::max(scratch[l], scratch_size(static_cast<iso_algorithm>(req[r].algorithm), items[r].g,
+                                                       items[r].pl.cp));
         if (out && req[r].algorithm == ISO_MARCHING_CUBES) {
             const long long capV = vertex_limit(&out[r], out[r].cap_points);
             const long long capM = capV < 0xffffffffll ? capV : 0xffffffffll;
@@ -469,11 +470,11 @@ void enqueue_batch(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, in
         BatchItem& it = items[r];
         cudaStream_t ls = ctx->lane_streams[it.lane];
         FeBuffers b;
-        carve(arena + lay.scratch_at[it.lane], it.g, it.pl.cp, b);
+        const iso_algorithm algo = static_cast<iso_algorithm>(req[r].algorithm);
+        carve(arena + lay.scratch_at[it.lane], algo, it.g, it.pl.cp, b);
         b.totals = counters + 8 * r;
         b.fe2mc = reinterpret_cast<uint32_t*>(arena + lay.map_at[it.lane]);
         PassMarks pm(ctx, ls);
-        const iso_algorithm algo = static_cast<iso_algorithm>(req[r].algorithm);
         enqueue_count(ctx, algo, req[r].volume, it.g, req[r].isoval, it.pl, b, ls, pm);
         if (out) enqueue_generate(ctx, algo, req[r].volume, it.g, req[r].isoval, it.pl, b, &out[r], ls, pm);
     }
@@ -945,7 +946,7 @@ iso_status iso_block_tris(iso_ctx* ctx, const float* volume, const iso_grid* gri
     ISO_CUDA(ctx, cudaSetDevice(ctx->device));
     const Plans pl = make_plans(ctx, g);
     FeBuffers b;
-    iso_status st = ensure_scratch(ctx, g, pl.cp, b, s);
+    iso_status st = ensure_scratch(ctx, ISO_FLYING_EDGES, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     iso::launch_count(volume, g, isoval, ctx->d_cases, false, pl.cp, b, s);  // bit rows of the whole grid
     ISO_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(int32_t) * (size_t)iso::block_count(g), s));

@@ -72,7 +72,7 @@ iso_status slab_count_enqueue(iso_ctx* ctx, iso_algorithm algo, const float* vol
     enqueue_count(ctx, algo, vol, g, iso, pl, b, s, pm, d);
     ISO_CUDA(ctx, cudaGetLastError());
     const long long rlo = (long long)(k0 - g.kr) * g.ny, rhi = (long long)(k1 - g.kr) * g.ny;
-    iso::launch_slab_readback(b, g, rlo, rhi, rlo > 0, k1 < g.nz, d + 4, s);
+    iso::launch_slab_readback(b, g, algo == ISO_MARCHING_CUBES ? 3 : 2, rlo, rhi, rlo > 0, k1 < g.nz, d + 4, s);
     ISO_CUDA(ctx, cudaGetLastError());
     return ISO_OK;
 }
@@ -166,7 +166,7 @@ iso_status slab_prepare(iso_ctx* ctx, iso_algorithm algo, const float* volume, c
         ctx->last_error = "slabs need rows of at most 1024 points";
         return ISO_ERR_INVALID_ARG;
     }
-    return ensure_scratch(ctx, g, pl.cp, b, s);
+    return ensure_scratch(ctx, algo, g, pl.cp, b, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -287,7 +287,7 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
         for (int q = 0; q < nslab; ++q) {
             Grid gq;
             if (!slab_grid(grid, algo, slab_k0(q), slab_k0(q + 1), gq)) return ISO_ERR_INVALID_ARG;
-            const size_t need = scratch_size(gq, make_plans(ctx, gq).cp);
+            const size_t need = scratch_size(algo, gq, make_plans(ctx, gq).cp);
             if (need > best) {
                 best = need;
                 qb = q;
@@ -297,8 +297,8 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
         if (!slab_grid(grid, algo, slab_k0(qb), slab_k0(qb + 1), gq)) return ISO_ERR_INVALID_ARG;
         const Plans pq = make_plans(ctx, gq);
         FeBuffers unused;
-        iso_status e = ensure_scratch(ctx, gq, pq.cp, unused, s);
-        if (e == ISO_OK) e = ensure_scratch_b(ctx, gq, pq.cp, unused, s);
+        iso_status e = ensure_scratch(ctx, algo, gq, pq.cp, unused, s);
+        if (e == ISO_OK) e = ensure_scratch_b(ctx, algo, gq, pq.cp, unused, s);
         if (e != ISO_OK) return e;
     }
     const char* src = static_cast<const char*>(volume);
@@ -365,7 +365,8 @@ iso_status extract_host_streamed(iso_ctx* ctx, iso_algorithm algo, const void* v
             iso::launch_to_float(typed_window(q), dtype, window(q),
                                  (long long)(data_hi(q) - data_lo(q) + 1) * (long long)plane, ctx->nsm, sc);
         iso_status e =
-            (q & 1) ? ensure_scratch_b(ctx, r.g, r.pl.cp, r.b, sc) : ensure_scratch(ctx, r.g, r.pl.cp, r.b, sc);
+            (q & 1) ? ensure_scratch_b(ctx, algo, r.g, r.pl.cp, r.b, sc)
+                    : ensure_scratch(ctx, algo, r.g, r.pl.cp, r.b, sc);
         if (e != ISO_OK) return e;
         e = slab_count_enqueue(ctx, algo, window(q), r.g, r.k0, r.k1, isoval, r.pl, r.b, sc,
                                ctx->h_slab + kSlabWords * (q & 1));
@@ -691,7 +692,7 @@ iso_status iso_count_device(iso_ctx* ctx, iso_algorithm algo, const float* volum
     ISO_CUDA(ctx, cudaSetDevice(ctx->device));
     const Plans pl = make_plans(ctx, g);
     FeBuffers b;
-    iso_status st = ensure_scratch(ctx, g, pl.cp, b, s);
+    iso_status st = ensure_scratch(ctx, algo, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     PassMarks pm(ctx, s);
     enqueue_count(ctx, algo, volume, g, isoval, pl, b, s, pm, ctx->h_totals);
@@ -722,7 +723,7 @@ static iso_status extract_device(iso_ctx* ctx, iso_algorithm algo, const float* 
         return ISO_ERR_INVALID_ARG;
     }
     FeBuffers b;
-    st = ensure_scratch(ctx, g, pl.cp, b, s);
+    st = ensure_scratch(ctx, algo, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     if (algo == ISO_MARCHING_CUBES) {
         st = ensure_fe2mc(ctx, out->cap_points, s);
@@ -802,7 +803,7 @@ static iso_status extract_host_impl(iso_ctx* ctx, iso_algorithm algo, const void
         return ISO_ERR_INVALID_ARG;
     }
     FeBuffers b;
-    st = ensure_scratch(ctx, g, pl.cp, b, s);
+    st = ensure_scratch(ctx, algo, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     PassMarks pm(ctx, s);
     enqueue_count(ctx, algo, ctx->d_volume, g, isoval, pl, b, s, pm, ctx->h_totals);
@@ -872,7 +873,7 @@ static iso_status extract_device_narrow(iso_ctx* ctx, iso_algorithm algo, const 
 {
     const Plans pl = make_plans(ctx, g);
     FeBuffers b;
-    iso_status st = ensure_scratch(ctx, g, pl.cp, b, s);
+    iso_status st = ensure_scratch(ctx, algo, g, pl.cp, b, s);
     if (st != ISO_OK) return st;
     const bool mc = algo == ISO_MARCHING_CUBES;
     const long long capV = vertex_limit(out, out->cap_points);
@@ -995,8 +996,8 @@ iso_status iso_fe_pass1(iso_fe* fe)
     const size_t vbytes = (size_t)g.nx * g.ny * g.nz * sizeof(float);
     const Plans pl = make_plans(ctx, g);
     ISO_CUDA(ctx, cudaMalloc(&fe->d_volume, vbytes));
-    ISO_CUDA(ctx, cudaMalloc(&fe->scratch, scratch_size(g, pl.cp)));
-    carve(fe->scratch, g, pl.cp, fe->buf);
+    ISO_CUDA(ctx, cudaMalloc(&fe->scratch, scratch_size(ISO_FLYING_EDGES, g, pl.cp, true)));
+    carve(fe->scratch, ISO_FLYING_EDGES, g, pl.cp, fe->buf, true);
     ISO_CUDA(ctx, cudaMemcpy(fe->d_volume, fe->host_volume, vbytes, cudaMemcpyHostToDevice));
     iso::CountPlan cp = pl.cp;
     cp.trims = true;  // the gridEdge records carry them

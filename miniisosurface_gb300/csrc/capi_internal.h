@@ -191,30 +191,55 @@ inline bool make_grid(const iso_grid* gr, Grid& g)
 
 inline bool empty_grid(const Grid& g) { return g.nx < 2 || g.ny < 2 || g.nz < 2; }
 
-inline size_t scratch_size(const Grid& g, const iso::CountPlan& cp)
+// What an extraction keeps per grid row: the starts of the components its scan sums (ScanMode, iso_kernels.h), the low
+// ids that k_gen_cells reads (not the duplicate-free order), the Marching Cubes counts, and the trims, which the
+// pass-by-pass object alone asks for. 48, 60 and 48 bytes a row for Flying Edges, Marching Cubes and the duplicate-free
+// order, and the bits.
+struct ScratchParts {
+    size_t comps;
+    bool row4, mccnt, trims;
+};
+inline ScratchParts scratch_parts(iso_algorithm algo, bool trims)
 {
-    const size_t R = (size_t)g.R;
-    return 2 * align256(R * 16) + align256(R * 8) + align256(R * 4) + align256(4 * R * 8) +
-           align256(4 * (size_t)cp.nseg * 8) + align256(8 * 8) + align256(R * (size_t)g.W * 4);
+    const bool mc = algo == ISO_MARCHING_CUBES, dup = algo == ISO_MC_DUPFREE;
+    return {(size_t)(dup ? 4 : (mc ? 3 : 2)), !dup, mc, trims};
 }
 
-inline void carve(void* base, const Grid& g, const iso::CountPlan& cp, FeBuffers& b)
+inline size_t scratch_size(iso_algorithm algo, const Grid& g, const iso::CountPlan& cp, bool trims = false)
 {
     const size_t R = (size_t)g.R;
+    const ScratchParts h = scratch_parts(algo, trims);
+    return align256(8 * 8) + align256(R * 16) + (h.row4 ? align256(R * 16) : 0) + (h.trims ? align256(R * 8) : 0) +
+           (h.mccnt ? align256(R * 4) : 0) + align256(h.comps * R * 8) + align256(h.comps * (size_t)cp.nseg * 8) +
+           align256(R * (size_t)g.W * 4);
+}
+
+inline void carve(void* base, iso_algorithm algo, const Grid& g, const iso::CountPlan& cp, FeBuffers& b,
+                  bool trims = false)
+{
+    const size_t R = (size_t)g.R;
+    const ScratchParts h = scratch_parts(algo, trims);
     char* p = static_cast<char*>(base);
-    b.totals = reinterpret_cast<unsigned long long*>(p); p += align256(8 * 8);
-    b.rowcnt = reinterpret_cast<uint4*>(p); p += align256(R * 16);
-    b.row4 = reinterpret_cast<uint4*>(p); p += align256(R * 16);
-    b.trims = reinterpret_cast<uint2*>(p); p += align256(R * 8);
-    b.mccnt = reinterpret_cast<uint32_t*>(p); p += align256(R * 4);
-    b.starts = reinterpret_cast<unsigned long long*>(p); p += align256(4 * R * 8);
-    b.part = reinterpret_cast<unsigned long long*>(p); p += align256(4 * (size_t)cp.nseg * 8);
-    b.bits = reinterpret_cast<uint32_t*>(p);
+    auto take = [&](bool held, size_t bytes) -> void* {
+        if (!held) return nullptr;
+        char* at = p;
+        p += align256(bytes);
+        return at;
+    };
+    b.totals = static_cast<unsigned long long*>(take(true, 8 * 8));
+    b.rowcnt = static_cast<uint4*>(take(true, R * 16));
+    b.row4 = static_cast<uint4*>(take(h.row4, R * 16));
+    b.trims = static_cast<uint2*>(take(h.trims, R * 8));
+    b.mccnt = static_cast<uint32_t*>(take(h.mccnt, R * 4));
+    b.starts = static_cast<unsigned long long*>(take(true, h.comps * R * 8));
+    b.part = static_cast<unsigned long long*>(take(true, h.comps * (size_t)cp.nseg * 8));
+    b.bits = static_cast<uint32_t*>(take(true, R * (size_t)g.W * 4));
 }
 
-inline iso_status ensure_scratch(iso_ctx* ctx, const Grid& g, const iso::CountPlan& cp, FeBuffers& b, cudaStream_t s)
+inline iso_status ensure_scratch(iso_ctx* ctx, iso_algorithm algo, const Grid& g, const iso::CountPlan& cp,
+                                 FeBuffers& b, cudaStream_t s)
 {
-    const size_t need = scratch_size(g, cp);
+    const size_t need = scratch_size(algo, g, cp);
     if (need > ctx->scratch_bytes) {
         if (ctx->scratch) {
             ISO_CUDA(ctx, cudaStreamSynchronize(s));
@@ -226,7 +251,7 @@ inline iso_status ensure_scratch(iso_ctx* ctx, const Grid& g, const iso::CountPl
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch, alloc));
         ctx->scratch_bytes = alloc;
     }
-    carve(ctx->scratch, g, cp, b);
+    carve(ctx->scratch, algo, g, cp, b);
     b.kept = ctx->d_status;
     b.fe2mc = ctx->fe2mc;
     return ISO_OK;
@@ -247,9 +272,10 @@ inline iso_status ensure_typed(iso_ctx* ctx, size_t bytes, cudaStream_t s)
 
 // The second scratch set (the streamed path counts slab q+1 while slab q
 // is generated from the first).
-inline iso_status ensure_scratch_b(iso_ctx* ctx, const Grid& g, const iso::CountPlan& cp, FeBuffers& b, cudaStream_t s)
+inline iso_status ensure_scratch_b(iso_ctx* ctx, iso_algorithm algo, const Grid& g, const iso::CountPlan& cp,
+                                   FeBuffers& b, cudaStream_t s)
 {
-    const size_t need = scratch_size(g, cp);
+    const size_t need = scratch_size(algo, g, cp);
     if (need > ctx->scratch_b_bytes) {
         if (ctx->scratch_b) {
             ISO_CUDA(ctx, cudaStreamSynchronize(s));
@@ -261,7 +287,7 @@ inline iso_status ensure_scratch_b(iso_ctx* ctx, const Grid& g, const iso::Count
         ISO_CUDA(ctx, cudaMalloc(&ctx->scratch_b, alloc));
         ctx->scratch_b_bytes = alloc;
     }
-    carve(ctx->scratch_b, g, cp, b);
+    carve(ctx->scratch_b, algo, g, cp, b);
     b.kept = ctx->d_status;
     b.fe2mc = ctx->fe2mc;
     return ISO_OK;

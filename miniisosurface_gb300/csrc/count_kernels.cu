@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) k_count_wide(const float* __restrict
 // kSeg rows (256 threads x 4):
 //   k_scan_partial  one CTA per segment: segment totals
 //   k_scan_final    one CTA per segment: offset of the segment + scan inside
-//                   it -> starts[3][R]; grand totals.
+//                   it -> starts[n][R]; grand totals.
 // ---------------------------------------------------------------------------
 constexpr int kScanPer = 4;  // 4 rather than 8 rows per thread: twice the CTAs, 15.2 -> 12.9 us at 512^3
 constexpr int kSeg = kThreads * kScanPer;
@@ -941,20 +941,20 @@ RowStarts row_starts(const Grid& g, const CountPlan& p, const FeBuffers& b)
 // one warp straight into mapped pinned host memory (no copy engine: the read-back
 // does not queue behind bulk copies of other streams): out[a] the start of row
 // rlo and out[3 + a] that of row rhi, for a = vertices, triangles, MC vertices.
-__global__ void k_slab_readback(const unsigned long long* __restrict__ starts, long long R, long long rlo,
+__global__ void k_slab_readback(const unsigned long long* __restrict__ starts, int comps, long long R, long long rlo,
                                 long long rhi, int has_lo, int has_hi, unsigned long long* out)
 {
     const int a = threadIdx.x;
     if (a < 3) {
-        if (has_lo) out[a] = starts[a * R + rlo];
-        if (has_hi) out[3 + a] = starts[a * R + rhi];
+        if (has_lo) out[a] = a < comps ? starts[a * R + rlo] : 0ull;
+        if (has_hi) out[3 + a] = a < comps ? starts[a * R + rhi] : 0ull;
     }
 }
 
-void launch_slab_readback(const FeBuffers& b, const Grid& g, long long rlo, long long rhi, bool has_lo, bool has_hi,
-                          unsigned long long* out, cudaStream_t s)
+void launch_slab_readback(const FeBuffers& b, const Grid& g, int comps, long long rlo, long long rhi, bool has_lo,
+                          bool has_hi, unsigned long long* out, cudaStream_t s)
 {
-    k_slab_readback<<<1, 32, 0, s>>>(b.starts, g.R, rlo, rhi, has_lo ? 1 : 0, has_hi ? 1 : 0, out);
+    k_slab_readback<<<1, 32, 0, s>>>(b.starts, comps, g.R, rlo, rhi, has_lo ? 1 : 0, has_hi ? 1 : 0, out);
 }
 
 void launch_grid_edges(const Grid& g, const CountPlan& p, const FeBuffers& b, int scanned, unsigned long long* ge,

@@ -17,11 +17,11 @@ struct RowStarts;
 // launchers).  R = ny*nz grid rows, W = ceil(nx/32) words per row.
 struct FeBuffers {
     uint4* rowcnt = nullptr;               // R      x/y/z cuts, triangles
-    uint4* row4 = nullptr;                 // R      low 32 bits of the row's first x, y and z cut's ids (scan)
-    uint2* trims = nullptr;                // R      xl, xr (pass 1 trims)
-    uint32_t* mccnt = nullptr;             // R      MC vertices per cell row
-    unsigned long long* starts = nullptr;  // 4*R    per row: first vertex, triangle, MC vertex (or y, z cuts)
-    unsigned long long* part = nullptr;    // 4*nseg scan segment totals
+    uint4* row4 = nullptr;                 // R      low 32 bits of the row's first x, y and z cut's ids (scan); not kScanDup
+    uint2* trims = nullptr;                // R      xl, xr (pass 1 trims); null unless the plan asks for them
+    uint32_t* mccnt = nullptr;             // R      MC vertices per cell row; kScanMC alone
+    unsigned long long* starts = nullptr;  // n*R    per row: first vertex, triangle, MC vertex (or y, z cuts); n components
+    unsigned long long* part = nullptr;    // n*nseg scan segment totals
     unsigned long long* totals = nullptr;  // 8      vertices, triangles, mc vertices, status, x cuts, y cuts, -, work counter
     uint32_t* bits = nullptr;              // R*W    bit rows
     unsigned long long* kept = nullptr;    // 1      device status of the calls that publish (count_status)
@@ -117,9 +117,9 @@ enum ScanMode { kScanFE = 0, kScanMC = 1, kScanDup = 2 };
 // the totals and the context's status word are also written there, and that word is zero again for the next count.
 void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cudaStream_t s,
                  unsigned long long* publish = nullptr);
-// the starts of rows rlo / rhi into out[0..5] (device-visible host memory)
-void launch_slab_readback(const FeBuffers& b, const Grid& g, long long rlo, long long rhi, bool has_lo, bool has_hi,
-                          unsigned long long* out, cudaStream_t s);
+// the starts of rows rlo / rhi into out[0..5] (device-visible host memory), zero for components past the scan's comps
+void launch_slab_readback(const FeBuffers& b, const Grid& g, int comps, long long rlo, long long rhi, bool has_lo,
+                          bool has_hi, unsigned long long* out, cudaStream_t s);
 // Marching Cubes in two passes (rows of up to 32 words, whole windows): owned
 // vertices and FE-id triangles together, then the triangles' ids remapped
 bool mc_fused(const Grid& g, const GenPlan& p);
