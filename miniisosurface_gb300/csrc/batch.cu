@@ -78,8 +78,9 @@ struct FusedPlan {
 // Bytes of n descriptors at the start of the upload block (the lists and firsts follow, 256-byte aligned).
 inline size_t desc_bytes(size_t n) { return (n * sizeof(iso::BatchReq) + 255) & ~(size_t)255; }
 
-// Fewest fusable requests that run fused by default (iso_batch_set_fused 1): serving batches of 2-8 requests
-// ran 4-8% faster on the lanes, the 157-request batch 11% faster fused.
+// Fewest fusable requests that run fused by default (iso_batch_set_fused 1). Time on the lanes over time fused, graphs
+// replayed: 64^3 volumes 0.47 (2 requests), 0.68 (8), 0.80 (16), 0.99 (24), 1.15 (32), 1.33 (64); volumes with sides in
+// [48, 200) 0.58 (2), 0.99 (8), 1.11 (12), 1.15 (16), 1.24 (32): the larger the volumes, the fewer requests it takes.
 constexpr int kFuseMin = 16;
 
 bool fusable(const iso_ctx* ctx, const iso_request& r, const BatchItem& it)
@@ -88,14 +89,16 @@ bool fusable(const iso_ctx* ctx, const iso_request& r, const BatchItem& it)
            (reinterpret_cast<uintptr_t>(r.volume) & 15) == 0;
 }
 
-// Groups, work split and layout of the fused requests fz (their plans are made for the whole GPU).  Returns
-// an empty plan when a launch would pass 2^31 blocks or items: those requests then take the lanes.
-// Work split of the fused launches: count blocks of at least kc planes, generate items for about ipw per warp
-// of one wave (the autotuner's candidates; 0: the defaults).
+// Work split of the fused launches: count blocks of at least kc planes, generate items for about ipw per kFusedWarps
+// warps of every SM (the autotuner's candidates; 0: the defaults).
 constexpr int kFusedKC[] = {8, 16, 32};
 constexpr int kFusedIPW[] = {16, 32, 64};
 constexpr int kFusedKCDefault = 16, kFusedIPWDefault = 16;
+// The unit in which ipw counts, no launch: the kernel runs 2 CTAs of up to 14 warps (gen_cells.cuh).
+constexpr int kFusedWarps = 32;
 
+// Groups, work split and layout of the fused requests fz (their plans are made for the whole GPU).  Returns
+// an empty plan when a launch would pass 2^31 blocks or items: those requests then take the lanes.
 FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, std::vector<BatchItem>& items,
                      const std::vector<int>& fz, const iso::PackedOut* pk = nullptr, int kc_min = 0, int ipw = 0)
 {
@@ -108,8 +111,8 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
     const int nf = (int)fz.size();
     f.proto.resize(nf);
     std::map<int, int> ckey, gkey;
-    const long long warps = (long long)ctx->nsm * 4 * 8;  // generate kernel: 4 CTAs of 8 warps per SM
-    long long gen_planes = 0;                              // row groups x planes over all generate groups
+    const long long warps = (long long)ctx->nsm * kFusedWarps;
+    long long gen_planes = 0;  // row groups x planes over all generate groups
     for (int d = 0; d < nf; ++d) {
         const int r = fz[d];
         BatchItem& it = items[r];
@@ -150,7 +153,7 @@ FusedPlan plan_fused(iso_ctx* ctx, const iso_request* req, const iso_mesh* out, 
             gen_planes += (long long)x.gen_ngroups * g.nz;
         }
     }
-    // generate items of KC planes: about ipw per warp of one wave over all requests, at least 2 planes
+    // generate items of KC planes: about ipw for each of the unit's warps, over all requests, at least 2 planes
     long long KC = (gen_planes + ipw * warps - 1) / (ipw * warps);
     if (KC < 2) KC = 2;
     const long long lim = 1ll << 31;

@@ -944,7 +944,7 @@ iso_status iso_extract_device_typed(iso_ctx* ctx, iso_algorithm algo, const void
         if (st != ISO_OK) return st;
         out->n_points = out->n_tris = 0;
         const Plans pl = make_plans(ctx, g);
-        if (pl.gp.fits && (algo == ISO_FLYING_EDGES || iso::mc_fused(g, pl.gp)))
+        if (pl.gp.fits)
             return extract_device_narrow(ctx, algo, volume, dtype, g, isoval, out, s);
     }
     const long long n = (long long)g.nx * g.ny * g.nz;

@@ -423,7 +423,7 @@ inline void enqueue_generate(iso_ctx* ctx, iso_algorithm algo, const float* vol,
             pm.mark(ISO_PASS_VERTICES);
     } else {
         const long long capM = capV < 0xffffffffll ? capV : 0xffffffffll;  // fe2mc holds 32-bit ids
-        if (pl.gp.fits && iso::mc_fused(g, pl.gp)) {  // owned vertices + FE-id triangles, vertices, remap
+        if (pl.gp.fits) {  // owned vertices + FE-id triangles, vertices, remap
             if (i4)
                 iso::launch_mc_gen_tris<uint32_t>(g, ctx->d_cases, b, pl.cp, pl.gp, capM, capT, out->points,
                                                   static_cast<uint32_t*>(out->tris), ctx->reverse, s);
@@ -440,30 +440,15 @@ inline void enqueue_generate(iso_ctx* ctx, iso_algorithm algo, const float* vol,
             pm.mark(ISO_PASS_MC_TRIANGLES);
             return;
         }
-        if (pl.gp.fits)
-            iso::launch_mc_gen_warps(vol, g, iso, ctx->d_cases, b, pl.cp, pl.gp, capM, capT, out->points, out->normals,
-                                     ctx->reverse, s);
-        else
-            iso::launch_mc_vertices_rows(vol, g, iso, ctx->d_cases, b, pl.cp, capM, capT, out->points, out->normals,
-                                         ctx->nsm, s);
+        iso::launch_mc_vertices_rows(vol, g, iso, ctx->d_cases, b, pl.cp, capM, capT, out->points, out->normals,
+                                     ctx->nsm, s);
         pm.mark(ISO_PASS_MC_VERTICES);
-        if (pl.gp.fits && iso::launch_mc_vertices(vol, g, iso, b, pl.gp, capM, capT, out->points, out->normals, s))
-            pm.mark(ISO_PASS_VERTICES);
-        if (pl.gp.fits) {
-            if (i4)
-                iso::launch_mc_tri_warps<uint32_t>(g, ctx->d_cases, b, pl.cp, pl.gp, capM, capT,
-                                                   static_cast<uint32_t*>(out->tris), s);
-            else
-                iso::launch_mc_tri_warps<uint64_t>(g, ctx->d_cases, b, pl.cp, pl.gp, capM, capT,
-                                                   static_cast<uint64_t*>(out->tris), s);
-        } else {
-            if (i4)
-                iso::launch_mc_triangles<uint32_t>(g, ctx->d_cases, b, pl.cp, capM, capT,
-                                                   static_cast<uint32_t*>(out->tris), ctx->nsm, s);
-            else
-                iso::launch_mc_triangles<uint64_t>(g, ctx->d_cases, b, pl.cp, capM, capT,
-                                                   static_cast<uint64_t*>(out->tris), ctx->nsm, s);
-        }
+        if (i4)
+            iso::launch_mc_triangles<uint32_t>(g, ctx->d_cases, b, pl.cp, capM, capT,
+                                               static_cast<uint32_t*>(out->tris), ctx->nsm, s);
+        else
+            iso::launch_mc_triangles<uint64_t>(g, ctx->d_cases, b, pl.cp, capM, capT,
+                                               static_cast<uint64_t*>(out->tris), ctx->nsm, s);
         pm.mark(ISO_PASS_MC_TRIANGLES);
     }
 }

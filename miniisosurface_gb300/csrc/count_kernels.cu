@@ -3,7 +3,7 @@
 // (cube cases, per-row counts):
 //
 //   k_count_rows   (rows up to 1024 points, the volume at a 16-byte boundary;
-//                  count_rows.cuh) a warp owns 1 to 128 neighbouring grid rows
+//                  count_rows.cuh) a warp owns 1 to 64 neighbouring grid rows
 //                  and a run of KC planes and marches along z, a bulk copy of
 //                  its rows of plane k+2 in flight while plane k is counted.
 //   k_count_warps  (up to 2048 points, any boundary) a CTA owns a block of 8
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(kThreads) k_count_warps(const float* __restric
 
 // Rows of up to 32 words, the volume at a 16-byte boundary (count_rows.cuh).  Against the kernel it replaced (lanes
 // per row a power of two, every row classified twice), us: 768^3 302 / 453, 667 x 228 x 724 94 / 152, 301 x 217 x 190
-// 18.6 / 32, 64^3 10 / 21; 512^3 104 / 103, both at the HBM rate (6.6 TB/s alone; in a sequence of extractions the
-// mesh written before drains at the same time).
+// 18.6 / 32, 64^3 10 / 21; 512^3 104 / 103, both at the HBM rate (the kernel by itself 88 us, 6.1 TB/s; in a sequence
+// of extractions the mesh written before drains at the same time).
 template <bool MC, int S, bool ALIGNED>
 __global__ void __launch_bounds__(kCountThreads) k_count_rows(const float* __restrict__ vol, Grid g, float below,
                                                               int KC, int ngroups, unsigned nitems, int stage_bytes,
@@ -525,7 +525,9 @@ __global__ void __launch_bounds__(kThreads) k_scan_final(const uint4* rowcnt,
 
 // The whole scan of a small grid in one CTA: one launch less than the two above where launches are most of the time.
 // A warp takes a run of 128 consecutive rows, a lane every 32nd of them, read once.  Events around the pass, us: 64^3
-// (4,096 rows) 9.0 against 11.4 with the two; at 16,384 rows (128^3) one CTA takes 18, the two 10.
+// (4,096 rows) 9.0 against 11.4 with the two.  The limit is where a thread's four rows end.  With sixteen, up to 16,384
+// rows, the call (rows of 64 points) takes longer at every size, us: 3,000 rows 44-48 (with four 40), 5,120 rows 46-49
+// (the two kernels 43), 8,000 rows 48-52 (45), 12,000 rows 53-56 (47), 16,384 rows 58-59 (49).
 constexpr int kScanSmallPer = 4;
 constexpr long long kScanSmall = 1024ll * kScanSmallPer;
 

@@ -4,8 +4,9 @@
 // vertices of every grid row.
 //
 // A row's W words go to W neighbouring lanes, 32 / W rows side by side in a
-// warp, so 94% of the lanes hold a word on average over the widths (powers of
-// two of lanes per row left a 5-word row 3 of 8 lanes idle).  A lane holds S
+// warp, so 91% of the lanes hold a word on average over the widths up to 16, 84%
+// up to 32 (powers of two of lanes per row left a 5-word row 3 of 8 lanes idle;
+// rows of 17 to 31 words leave 32 - W idle either way).  A lane holds S
 // consecutive rows of its place plus the row after them: a warp's rows are
 // jw .. jw + G - 1, G = (32 / W) * S, and they read rows jw .. jw + G of every
 // plane, which lie next to each other in memory, so one bulk copy per plane
@@ -219,7 +220,9 @@ __device__ __forceinline__ void count_rows_item(const typename Samples::T* __res
             long long a0, e1;
             const long long e = extent(s0, a0, e1);
             at += (int)(s0 - a0);
-            if (e1 < e) {  // the last points of the pass' last plane
+            // the last points of the pass' last plane. No copy into these bytes follows: the planes after it, which there
+            // are only where a plane has fewer than PER points, end in the same 16 bytes and copy nothing.
+            if (e1 < e) {
                 if (lane < (int)(e - e1)) reinterpret_cast<T*>(buf)[(int)(e1 - a0) + lane] = __ldg(vol + e1 + lane);
                 __syncwarp();
             }

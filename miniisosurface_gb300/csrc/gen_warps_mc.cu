@@ -62,8 +62,6 @@ bool launch_dup_vertices(const float* vol, const Grid& g, float iso, const FeBuf
 // vertices (records, FE -> MC map) and the triangles with the corners' Flying
 // Edges ids in one generate pass, then k_mc_remap replaces every index by its MC
 // id once the map is complete.
-bool mc_fused(const Grid& g, const GenPlan& p) { return p.nsm > 0 && p.kemit == g.kr; }
-
 template <typename IndexT>
 void launch_mc_gen_tris(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                         const GenPlan& p, long long capV, long long capT, float* points, IndexT* tris, int reverse,

@@ -4,13 +4,18 @@
 //   volume  float32[nz][ny][nx]                  x fastest (Image3D.h:26-85)
 //   rowcnt  uint4[R]       per grid row r = k*ny + j (R = ny*nz): cut x / y / z
 //                          edges owned by the row, triangles of cell row (j,k)
-//   trims   uint2[R]       xl, xr of the row (FlyingEdgesAlgorithm.cpp:47-65)
+//   row4    uint4[R]       low 32 bits of the ids of the row's first x, y and z
+//                          cut (not the duplicate-free order)
+//   trims   uint2[R]       xl, xr of the row (FlyingEdgesAlgorithm.cpp:47-65),
+//                          pass-by-pass interface only
 //   mccnt   uint32[R]      marching cubes: vertices owned by cell row (j,k)
-//   starts  u64[3][R]      first vertex / triangle / mc vertex of each row
-//                          (exclusive scans of the counts in row order)
+//   starts  u64[n][R]      first vertex / triangle / mc vertex of each row
+//                          (exclusive scans of the counts in row order): n = 2,
+//                          marching cubes 3, duplicate-free order 4 (first x cut,
+//                          triangle, y cut, z cut)
 //   bits    uint32[R][W]   W = ceil(nx/32); bit i of row r = value >= isovalue
-//                          (written only when a row-wise kernel needs it)
-//   totals  u64[4]         vertices, triangles, mc vertices, device status
+//   totals  u64[8]         vertices, triangles, mc vertices, device status, all
+//                          x cuts, all y cuts, -, work counter of pass 4
 //
 // All interpolation arithmetic goes through the _rn intrinsics so that no
 // multiply-add is ever contracted: that reproduces the float32 results of the
@@ -270,23 +275,6 @@ __device__ __forceinline__ unsigned long long fe_edge_id(const CutMasks& m, cons
                                 : sel == 4 ? b.yA : sel == 5 ? b.yC : sel == 6 ? b.zA : b.zB;
     return bs + __popc(mk & lowmask(bit + off));
 }
-
-// Walks the flattened index f = tid, tid + step, tid + 2*step, ... of a
-// (row, column) grid with `ncol` columns without dividing in the loop.
-struct RowColWalk {
-    int row, col, drow, dcol, ncol;
-    __device__ __forceinline__ RowColWalk(int start, int step, int ncol_)
-        : row(start / ncol_), col(start % ncol_), drow(step / ncol_), dcol(step % ncol_), ncol(ncol_) {}
-    __device__ __forceinline__ void advance()
-    {
-        row += drow;
-        col += dcol;
-        if (col >= ncol) {
-            col -= ncol;
-            ++row;
-        }
-    }
-};
 
 // Low grid point and axis of cube edge e of cell (0,0,0).
 __device__ __forceinline__ void cube_edge_geometry(int e, int& dx, int& dy, int& dz, int& axis)

@@ -120,9 +120,8 @@ void launch_scan(const Grid& g, const CountPlan& p, int mode, FeBuffers& b, cuda
 // the starts of rows rlo / rhi into out[0..5] (device-visible host memory), zero for components past the scan's comps
 void launch_slab_readback(const FeBuffers& b, const Grid& g, int comps, long long rlo, long long rhi, bool has_lo,
                           bool has_hi, unsigned long long* out, cudaStream_t s);
-// Marching Cubes in two passes (rows of up to 32 words, whole windows): owned
+// Marching Cubes in two passes (rows of up to 32 words, whole grids): owned
 // vertices and FE-id triangles together, then the triangles' ids remapped
-bool mc_fused(const Grid& g, const GenPlan& p);
 template <typename IndexT>
 void launch_mc_gen_tris(const Grid& g, const CaseTables* cases, const FeBuffers& b, const CountPlan& cp,
                         const GenPlan& p, long long capV, long long capT, float* points, IndexT* tris, int reverse,
@@ -167,6 +166,7 @@ bool launch_mc_vertices(const float* vol, const Grid& g, float iso, const FeBuff
 // The duplicate-free order's vertices from the records launch_dup_gen_warps wrote (whole grids)
 bool launch_dup_vertices(const float* vol, const Grid& g, float iso, const FeBuffers& b, const GenPlan& p,
                          long long capV, long long capT, float* points, float* normals, cudaStream_t s);
+// Marching Cubes of a slab in three: owned vertices and the map, the vertices, the triangles through the map
 void launch_mc_gen_warps(const float* vol, const Grid& g, float iso, const CaseTables* cases, const FeBuffers& b,
                          const CountPlan& cp, const GenPlan& p, long long capV, long long capT, float* points,
                          float* normals, int reverse, cudaStream_t s);

@@ -192,7 +192,7 @@ __global__ void k_block_tris(const uint32_t* __restrict__ bits, Grid g, BlockDim
 // 16-byte loads of four samples, two samples per instruction, in registers over
 // all tiles of the CTA; eight CTAs of a cluster then add theirs up through
 // distributed shared memory, so that a gradient gets one global addition per
-// cluster instead of one per CTA (1.6 million on 6,401 addresses for 16,384
+// cluster instead of one per CTA (1.7 million on 6,465 addresses for 16,384
 // samples).  Sums are fused multiply-adds.
 // What bounds it, for 16,384 samples (256 tiles; 34 us, 38 with 512 threads of 4 x
 // 2, 106 with a row of 16 units per thread and every CTA's own additions): the
