@@ -4,7 +4,12 @@
 //
 // A new array of tens of megabytes has no pages yet; the copy back would bring
 // them in one by one, on one thread, which clears each: 2.4 ms for the 52 MB mesh
-// of a 256^3 noise volume, against 0.3 ms for the copy itself.
+// of a 256^3 noise volume, against 0.3 ms for the copy itself.  Memory that the
+// allocator kept from an earlier array has its pages already (arrays of up to
+// some 30 MB, call after call): what is missing is looked up first, and nothing is
+// done for less than a piece (extract of 120^3 noise, 21 MB, again and again: 382 us
+// with the faults of the first call only, 473 with helpers for pages that were
+// there, 331 now; every mesh kept: 1,386, 766, 696).
 //
 // The helper threads live for one call and come from one budget for the whole
 // process: callers on many threads share it instead of bringing up a team each,
@@ -53,6 +58,20 @@ struct Pieces {
         uintptr_t a = 0, e = 0;
         return pages(r, a, e) ? (int64_t)((e - a + piece - 1) / piece) : 0;
     }
+    // Bytes of range r without a page, counted up to `enough`; 0 where the system cannot say.
+    uintptr_t missing(int64_t r, uintptr_t enough) const
+    {
+        unsigned char present[4096];  // of 16 MB or more at a time
+        uintptr_t a = 0, e = 0, n = 0;
+        if (!pages(r, a, e)) return 0;
+        for (uintptr_t p = a; p < e && n < enough;) {
+            const uintptr_t most = sizeof present * page, len = e - p < most ? e - p : most;
+            if (mincore(reinterpret_cast<void*>(p), len, present) != 0) return 0;
+            for (uintptr_t q = 0; q < len / page; ++q) n += present[q] & 1 ? 0 : page;
+            p += len;
+        }
+        return n;
+    }
     // A thread's share: pieces in ascending order, so that one walk over the ranges finds them all.
     void work()
     {
@@ -98,9 +117,11 @@ iso_status iso_populate_host(int64_t n, void* const* ptrs, const int64_t* bytes)
     p.bytes = bytes;
     p.page = (uintptr_t)sysconf(_SC_PAGESIZE);
     p.piece = 1u << 20 > p.page ? 1u << 20 : p.page;  // a multiple of the page, cleared by one thread
-    int64_t total = 0;
-    for (int64_t r = 0; r < n; ++r) total += p.count(r);
-    const int helpers = take_helpers(total - 1);
+    const uintptr_t enough = (kMaxHelpers + 1) * p.piece;  // a piece for every thread
+    uintptr_t missing = 0;
+    for (int64_t r = 0; r < n && missing < enough; ++r) missing += p.missing(r, enough);
+    if (missing < p.piece) return ISO_OK;
+    const int helpers = take_helpers((int64_t)(missing / p.piece) - 1);
     std::thread team[kMaxHelpers];
     int made = 0;
     try {

@@ -73,3 +73,21 @@ resource.setrlimit(resource.RLIMIT_AS, (now + (2 << 20), resource.RLIM_INFINITY)
 assert populate(at, 64) == 0
 assert resident() - rss >= 60 << 20
 """)
+
+
+def test_present_pages_cost_no_thread(built):
+    """Memory that has its pages already (an array from memory the allocator kept): no helper is made.  Thread ids
+    count up, so that helpers between two threads' ids show; other processes may take some now and then."""
+    run(built, """
+def id_now():
+    t = threading.Thread(target=lambda: None)
+    t.start(); t.join()
+    return t.native_id
+def between(at):
+    a = id_now()
+    assert populate(at, 64) == 0
+    return id_now() - a
+m, at = fresh(64)
+assert between(at) > 1  # without pages: helpers
+assert min(between(at) for _ in range(20)) == 1
+""")
