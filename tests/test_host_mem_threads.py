@@ -18,7 +18,7 @@ def settled(n):  # a joined thread's entry may outlive the join by a moment
     while threads() > n and time.time() < end: time.sleep(0.01)
     return threads() <= n
 def fresh(mb):  # an anonymous mapping without pages
-    m = mmap.mmap(-1, mb << 20)
+    m = mmap.mmap(-1, mb << 20, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
     return m, C.addressof(C.c_char.from_buffer(m))
 def resident():
     return int(open("/proc/self/statm").read().split()[1]) * mmap.PAGESIZE
